@@ -48,3 +48,29 @@ def test_partial_pivoting_and_singular_warning():
     S = np.array([[1.0, 2.0], [2.0, 4.0]])
     with pytest.warns(RuntimeWarning):
         pfblob.lu_factor(S)
+
+
+@pytest.mark.parametrize("n", [2, 8, 32, 33, 64, 255, 257, 511, 513, 900, 1023, 1025, 2047, 2049])
+def test_lu_at_panel_edges_within_the_rounding_bound(n):
+    """P A = L U to the a priori bound of Gaussian elimination,
+    |PA - LU| <= 2 n u |L||U| elementwise (u = 2^-53, any order of the sums),
+    with |L| <= 1 (partial pivoting), at the sizes where the panel kernels
+    change; the same bound for the two substitutions' residual."""
+    import pfblob
+    rng = np.random.default_rng(1000 + n)
+    A = rng.standard_normal((n, n))
+    A[:, rng.permutation(n)[: n // 3]] *= 1e-3
+    b = rng.standard_normal(n)
+    lu, piv = pfblob.lu_factor(A)
+    P = np.arange(n)
+    for k in range(n):
+        assert k <= piv[k] < n
+        P[[k, piv[k]]] = P[[piv[k], k]]
+    L, U = np.tril(lu, -1) + np.eye(n), np.triu(lu)
+    assert np.abs(L).max() <= 1.0
+    u = 2.0 ** -53
+    LU = np.abs(L) @ np.abs(U)
+    assert (np.abs(A[P] - L @ U) <= 4 * n * u * LU).all()  # 2 n u, and as much for numpy's product
+    x = pfblob.lu_solve((lu, piv), b)
+    r = np.abs(A @ x - b)[P]
+    assert (r <= 8 * n * u * (LU @ np.abs(x)) + 4 * n * u * np.abs(b)[P]).all()
