@@ -187,6 +187,48 @@ __device__ __forceinline__ void pair2_far(const ulonglong2 &hi, const ulonglong2
     ny = fma2(dx, s, ny);
 }
 
+// ---------------------------------------------------------------------------
+// Which sources a run of targets needs not see in full: the bounding box of
+// the run's targets (hi parts of their coordinates) and a distance beyond
+// which every pair's r2 exceeds a bound whatever the rounding.  A source whose
+// hi part lies at box distance d has r2 >= (d - e)^2 for every target, e
+// covering the rounding of both hi parts (2^-23 relative each).
+struct TargetBox {
+    float x0, x1, y0, y1;
+    float reach2;  // (distance + margin)^2; infinite if a target is not finite
+};
+
+// Box of the warp's targets (valid: this lane has one); r2_min: the bound.
+__device__ __forceinline__ TargetBox warp_target_box(bool valid, float xh, float yh, float r2_min) {
+    TargetBox b;
+    b.x0 = valid ? xh : INFINITY;
+    b.x1 = valid ? xh : -INFINITY;
+    b.y0 = valid ? yh : INFINITY;
+    b.y1 = valid ? yh : -INFINITY;
+    const bool bad = __any_sync(0xffffffffu, valid && !isfinite(xh + yh));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        b.x0 = fminf(b.x0, __shfl_xor_sync(0xffffffffu, b.x0, o));
+        b.x1 = fmaxf(b.x1, __shfl_xor_sync(0xffffffffu, b.x1, o));
+        b.y0 = fminf(b.y0, __shfl_xor_sync(0xffffffffu, b.y0, o));
+        b.y1 = fmaxf(b.y1, __shfl_xor_sync(0xffffffffu, b.y1, o));
+    }
+    const float mag = fmaxf(fmaxf(fabsf(b.x0), fabsf(b.x1)), fmaxf(fabsf(b.y0), fabsf(b.y1)));
+    const float r = sqrtf(r2_min);
+    const float reach = r * 1.001f + (mag + r) * 4.8e-7f + 1e-30f;
+    // no target at all: beyond every source's reach (the box is inverted)
+    b.reach2 = bad ? INFINITY : (b.x0 <= b.x1 ? reach * reach : 0.f);
+    return b;
+}
+
+// True when the finite source (xh, yh, g) lies beyond the box's reach; a source
+// that is not finite never does (its NaN or infinity reaches every target).
+__device__ __forceinline__ bool beyond_reach(const TargetBox &b, float xh, float yh, float g) {
+    const float ex = fmaxf(fmaxf(b.x0 - xh, xh - b.x1), 0.f);
+    const float ey = fmaxf(fmaxf(b.y0 - yh, yh - b.y1), 0.f);
+    return fmaf(ex, ex, ey * ey) > b.reach2 && isfinite(xh + yh + g);
+}
+
 // Cutoff (Rosenhead-Krasny) kernel of the reference's vv2par
 // (src/cpp/blobs/c/vv2par_C/vv2par_C_cpu.c:143-148): s = g / (r^2 + sigma^2),
 // nx += dy*s, ny += dx*s; s2 = {sigma^2, sigma^2}.  The pair2_far arithmetic

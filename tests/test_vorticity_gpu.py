@@ -56,3 +56,33 @@ def test_empty_and_options():
     assert np.array_equal(w, np.zeros(3))
     with pytest.raises(Exception):
         pfblob.vorticity(np.ones(3), np.ones(3), np.ones(3), 0.01, method=0)
+
+
+@pytest.mark.parametrize("n,order", [(33, "lattice"), (257, "lattice"), (5000, "lattice"),
+                                     (20164, "lattice"), (5000, "random"), (5000, "clusters")])
+def test_sources_beyond_reach_add_nothing(n, order):
+    """Sources out of the exponential's FP32 range are skipped: lattice order
+    (most chunks skipped), random order (none), two clusters far apart (all of
+    the other one) against the FP64 oracle, 1e-6 as above; and a source that
+    is not finite still reaches every target."""
+    import pfblob
+    rng = np.random.default_rng(n)
+    s = int(np.sqrt(n))
+    h = 2.0 / max(s, 2)
+    if order == "lattice":
+        c = -1.0 + (np.arange(s) + 0.5) * h
+        x, y = (a.ravel().copy() for a in np.meshgrid(c, c, indexing="ij"))
+    else:
+        x, y = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+        if order == "clusters":
+            x[n // 2:] += 50.0
+            x[: n // 2] *= 0.1
+    g = rng.standard_normal(x.size) / x.size
+    sigma = h / 0.8
+    w = pfblob.vorticity(x, y, g, sigma)
+    assert err(w, oracle.vorticity_direct(x, y, g, 2 * sigma * sigma, x, y)) <= TOL
+    for bad in (np.nan, np.inf):
+        gb = g.copy()
+        gb[x.size // 3] = bad
+        assert np.isnan(pfblob.vorticity(x, y, gb, sigma, xEval=np.array([900.0]),
+                                         yEval=np.array([-900.0]))).all()
