@@ -65,6 +65,12 @@ constexpr int P2P_BUF = 64;      // sources per warp buffer (three buffers)
 constexpr int P2P_UNROLL = 8;
 constexpr int P2P_MIN_CTAS = 20; // one-warp CTAs resident per SM: 96 registers each
 constexpr unsigned INVALID_KEY = 0xFFFFFFFFu;
+// leaves of more particles than this are put in index order by the segment
+// sort; smaller ones by k_gather_sorted itself, c comparisons per particle.  A
+// layer around a body fills its leaves to 40-110 particles (the leaf level
+// comes from the blob count, the box is mostly empty); 1.8e6 blobs in an
+// annulus, gather + segment sort: 286 us at 64, 40 us at 256.
+constexpr int LEAF_SMALL = 256;
 
 // ---------------------------------------------------------------------------
 // Morton helpers (x in even bits, y in odd bits)
@@ -214,9 +220,9 @@ k_place(int64_t n, const uint32_t *__restrict__ key, const int32_t *__restrict__
     if (i >= n) return;
     const int64_t p = (int64_t)start[key[i]] + rank[i];
     if (PF_IDX_OK(p, n, 201)) perm[p] = (int32_t)i;
-    // a leaf of more than SEG_SMALL particles (exactly one has this rank) is
+    // a leaf of more than LEAF_SMALL particles (exactly one has this rank) is
     // listed for the segment sort
-    if (rank[i] == pf::SEG_SMALL) big[atomicAdd(big_n, 1)] = (int32_t)key[i];
+    if (rank[i] == LEAF_SMALL) big[atomicAdd(big_n, 1)] = (int32_t)key[i];
 }
 
 __host__ __device__ __forceinline__ int64_t level_off(int l) {
@@ -228,7 +234,7 @@ __host__ __device__ __forceinline__ int64_t level_off(int l) {
 // every later sum's order).  Thread j takes the particle i = perm[j] that the
 // counting sort placed in its leaf's range [s0, s0 + c); its final position
 // is s0 + (number of the leaf's particles with a smaller index), found by
-// reading the leaf's c entries of perm (leaves above SEG_SMALL particles are
+// reading the leaf's c entries of perm (leaves above LEAF_SMALL particles are
 // already in index order: seg_sort_listed).  Writes the final permutation to
 // perm_out and, at that position, FP64 x, y (g), the hi/lo float4 and float g
 // of the near field and the leaf key.
@@ -248,7 +254,7 @@ k_gather_sorted(int64_t n, const int32_t *__restrict__ perm, const uint32_t *__r
     const double gi = g ? g[i] : 0.0;
     const int s0 = start[m], c = cnt[m];
     int64_t d = j;
-    if (c <= pf::SEG_SMALL && PF_IDX_OK((int64_t)s0 + c - 1, n, 206)) {
+    if (c <= LEAF_SMALL && PF_IDX_OK((int64_t)s0 + c - 1, n, 206)) {
         int r = 0;
         for (int q = 0; q < c; ++q) r += perm[s0 + q] < i;
         d = (int64_t)s0 + r;
@@ -1594,9 +1600,9 @@ static pf_status sort_points(int64_t n, const double *x, const double *y,
     PF_CUDA_TRY(cudaMemsetAsync(big_n, 0, sizeof(int32_t), st));
     k_place<<<gn, 256, 0, st>>>(n, s.key, s.rank, s.start, s.perm, big, big_n);
     PF_TRY(pf::launch_status("k_place"));
-    // leaves above SEG_SMALL particles (dense clusters); the ranks are free now
+    // leaves above LEAF_SMALL particles (dense clusters); the ranks are free now
     PF_TRY(pf::seg_sort_listed(big, big_n, s.start, s.cnt, s.perm, s.rank,
-                               n / (pf::SEG_SMALL + 1) + 1, st));
+                               n / (LEAF_SMALL + 1) + 1, st));
     // the ranks are free again: they receive the final permutation
     k_gather_sorted<<<gn, 256, 0, st>>>(n, s.perm, s.key, s.start, s.cnt, x, y, g, s.rank, s.x,
                                         s.y, s.g, s.hl, s.g32, skey);
@@ -1641,7 +1647,7 @@ static size_t fmm_scratch_bytes(const FmmCache &c, int64_t ns, int64_t nt, bool 
     add(4 * nleaf); add(4 * nleaf);                 // starts src, tgt
     add(16 * (size_t)nbox * NP); add(16 * (size_t)nbox * NP);  // M, L
     add(16 * nt);                                   // near velocities
-    add(4 * (std::max(ns, nt) / (pf::SEG_SMALL + 1) + 3));  // leaves for the segment sort
+    add(4 * (std::max(ns, nt) / (LEAF_SMALL + 1) + 3));  // leaves for the segment sort
     add(4 * (64 + 2 * ((size_t)1 << (2 * (c.L - c.kb)))));  // P2P work distribution
     add(4 * pf::scan_tmp_ints(nleaf));
     return need + 4096;
@@ -1690,7 +1696,7 @@ static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, dou
     double2 *Lc = (double2 *)take(16 * (size_t)nbox * NP);
     double2 *nearv = (double2 *)take(16 * nt);
     // leaves listed for the segment sort: [0] count, [1 ..] leaf ids
-    int32_t *big = (int32_t *)take(4 * (std::max(ns, nt) / (pf::SEG_SMALL + 1) + 3));
+    int32_t *big = (int32_t *)take(4 * (std::max(ns, nt) / (LEAF_SMALL + 1) + 3));
     // P2P work distribution: counters (64 words), heavy list, group counters
     const int64_t nblk_w = (int64_t)1 << (2 * (L - kb));
     const size_t p2pw_bytes = 4 * (64 + 2 * (size_t)nblk_w);

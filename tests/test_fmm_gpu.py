@@ -229,3 +229,21 @@ def test_every_expansion_order_vs_oracle(terms, sigma):
     sub = np.arange(0, n, 15)
     rx, ry = oracle.velocity_direct(x, y, g, 2 * sigma * sigma, x[sub].copy(), y[sub].copy())
     assert normwise_err(vx[sub], vy[sub], rx, ry) <= TOL
+
+
+@pytest.mark.parametrize("k", [64, 65, 255, 256, 257, 300])
+def test_leaf_sizes_around_the_segment_sort(k):
+    """One leaf of k blobs among a uniform set (the leaf order changes from the
+    gather's own ranks to the segment sort above 256): against the oracle, and
+    the leaf's order is by input index, so a second call is bitwise the first."""
+    n = 6000
+    rng = np.random.default_rng(k)
+    x, y = rng.random(n), rng.random(n)
+    sel = rng.permutation(n)[:k]
+    x[sel] = 0.5 + 1e-3 * rng.random(k)
+    y[sel] = 0.5 + 1e-3 * rng.random(k)
+    g = rng.standard_normal(n) / n
+    a, b = fmm(x, y, g, 0.004), fmm(x, y, g, 0.004)
+    assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
+    rx, ry = oracle.velocity_direct(x, y, g, 2 * 0.004 ** 2)
+    assert normwise_err(*a, rx, ry) <= TOL
