@@ -43,6 +43,7 @@
 #include "fmm_api.cuh"
 #include "fmm_plan.cuh"
 #include "gauss_pair.cuh"
+#include "p2p.cuh"
 #include "scan.cuh"
 #include "segsort.cuh"
 
@@ -50,20 +51,11 @@
 
 namespace {
 
-using pf::fmmx::P2PDesc;
-using pf::fmmx::P2PWork;
-
 constexpr double THETA = 0.5;
 constexpr double INV_2PI = 0.15915494309189535;
 constexpr int MAX_LEVEL = pf::fmmx::MAX_LEVEL;
 constexpr int P2P_SETUP_THREADS = 128;
 constexpr int P2P_QMAX = 1024;   // source leaves per P2P block
-constexpr int P2P_RUNS_SM = 64;  // runs staged in shared memory at a time
-constexpr int P2P_BUF = 64;      // sources per warp buffer (three buffers)
-// unroll of the pair loop over a full chunk: the kernel holds nine copies of
-// it (targets per lane x mode), which must stay within the instruction cache
-constexpr int P2P_UNROLL = 8;
-constexpr int P2P_MIN_CTAS = 20; // one-warp CTAs resident per SM: 96 registers each
 constexpr unsigned INVALID_KEY = 0xFFFFFFFFu;
 // leaves of more particles than this are put in index order by the segment
 // sort; smaller ones by k_gather_sorted itself, c comparisons per particle.  A
@@ -753,577 +745,38 @@ k_p2p_runs(int L, int kb, const int2 *__restrict__ q, int nq, int nqp,
     if (!runs && threadIdx.x == 0) nruns_or_off[b] = s_n;
 }
 
-// P2P near field: one warp (one CTA) per P2P block, its targets in balanced
-// groups of at most 96.  Targets a and b of a lane run packed (f32x2); in a
-// group of 65..96 the remaining targets are spread over the warp, each lane
-// taking a share of the sources (p2p_split_sums).  Pair code modes, chosen
-// per source from its box distance to the group's target box (with a
-// rounding margin):
-//   P2P_FAR:    sources beyond sqrt(r2_far): no ex2 (1 - exp(-x) rounds to
-//               1.0f for every pair), one-float coordinates relative to the
-//               group centre;
-//   P2P_FULL:   the other sources beyond the series radius sqrt(r2_series):
-//               no small-x check (every pair has r2 above r2_series);
-//   P2P_SERIES: the sources within it: the pair code with the check.
-// Full and series pairs give bitwise the value of the checked code.  The group's
-// sources stream through three warp buffers, one per mode (each in stream
-// order), and each buffer runs 32 sources at a time as it fills (the rest
-// when the group's stream ends).
-constexpr int P2P_FAR = 0, P2P_FULL = 1, P2P_SERIES = 2;
-
-template <int MODE>
-__device__ __forceinline__ void scalar_pair(const ulonglong2 &h, const ulonglong2 &l,
-                                            unsigned long long g2, const float4 &t,
-                                            const pfd::GaussParams &gp, float &px, float &py) {
-    float sxh, syh, sxl, syl, g, dummy;
-    pfd::unpack2(h.x, sxh, dummy);
-    pfd::unpack2(h.y, syh, dummy);
-    pfd::unpack2(l.x, sxl, dummy);
-    pfd::unpack2(l.y, syl, dummy);
-    pfd::unpack2(g2, g, dummy);
-    const float dx = (t.x - sxh) + (t.z - sxl);
-    const float dy = (t.y - syh) + (t.w - syl);
-    const float r2 = fmaf(dx, dx, fmaf(dy, dy, 1e-12f));
-    const float sc = MODE == P2P_FAR ? g * pfd::rcp_approx(r2)
-                                     : pfd::gauss_s<MODE == P2P_SERIES>(r2, g, gp);
-    px = fmaf(-dy, sc, px);
-    py = fmaf(dx, sc, py);
-}
-
-// One pair of the given mode for the lane's targets (NT per lane).
-template <int NT, int MODE>
-__device__ __forceinline__ void p2p_pair(const ulonglong2 &h, const ulonglong2 &l,
-                                         unsigned long long g2, pfd::f32x2 txh, pfd::f32x2 tyh,
-                                         pfd::f32x2 txl, pfd::f32x2 tyl, const float4 &ta,
-                                         const float4 &tc, const pfd::GaussParams &gp,
-                                         const pfd::GaussParams2 &gp2, pfd::f32x2 &nx,
-                                         pfd::f32x2 &ny, float &pxa, float &pya, float &pxc,
-                                         float &pyc) {
-    if (NT >= 2) {
-        if (MODE == P2P_FAR)
-            pfd::pair2_far(h, l, g2, txh, tyh, txl, tyl, gp2, nx, ny);
-        else
-            pfd::pair2<MODE == P2P_SERIES>(h, l, g2, txh, tyh, txl, tyl, gp2, nx, ny);
-    } else {
-        scalar_pair<MODE>(h, l, g2, ta, gp, pxa, pya);
-    }
-    if (NT == 3) scalar_pair<MODE>(h, l, g2, tc, gp, pxc, pyc);
-}
-
-// Shared-memory loads by 32-bit shared address (the chunk functions below
-// are separate calls, which see only generic pointers otherwise).
-__device__ __forceinline__ ulonglong2 lds_u64x2(uint32_t a) {
-    ulonglong2 v;
-    asm("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "r"(a));
-    return v;
-}
-__device__ __forceinline__ unsigned long long lds_u64(uint32_t a) {
-    unsigned long long v;
-    asm("ld.shared.u64 %0, [%1];" : "=l"(v) : "r"(a));
-    return v;
-}
-
-struct P2PSums {
-    float s[6];  // NT >= 2: -nx_a, ny_a, -nx_b, ny_b; NT = 1: px_a, py_a; NT = 3: px_c, py_c
-};
-
-// Sources [0, cnt) of a buffer (cnt <= 32) against the lane's targets; the
-// partial sums are returned for one compensated fold by the caller.  Each
-// (NT, MODE) is its own function, not inlined: nine inlined copies of the
-// unrolled loop in one kernel measured about 20% more instructions (register
-// copies between the copies' allocations) and instruction-cache stalls.
-// (A per-source choice of the checked code inside a chunk, by a warp-uniform
-// branch, measured slower too: the branch breaks the overlap of consecutive
-// pairs.)
-//
-// P2P_FAR chunks hold coordinates relative to the group centre (cx, cy), one
-// float each: {x - cx, x - cx, y - cy, y - cy} in the hi slot (pair2_far_local).
-__device__ __forceinline__ void far_local_scalar(const ulonglong2 &loc, unsigned long long g2,
-                                                 float tx, float ty, float &px, float &py) {
-    float lx, ly, g, dummy;
-    pfd::unpack2(loc.x, lx, dummy);
-    pfd::unpack2(loc.y, ly, dummy);
-    pfd::unpack2(g2, g, dummy);
-    const float dx = tx - lx, dy = ty - ly;
-    const float r2 = fmaf(dx, dx, fmaf(dy, dy, 1e-12f));
-    const float sc = g * pfd::rcp_approx(r2);
-    px = fmaf(-dy, sc, px);
-    py = fmaf(dx, sc, py);
-}
-
-template <int NT, int MODE>
-__device__ __noinline__ P2PSums p2p_chunk_sums(uint32_t a_hi, uint32_t a_lo, uint32_t a_g, int cnt,
-                                               float4 ta, float4 tb, float4 tc, float cx,
-                                               float cy, pfd::GaussParams gp) {
-    const pfd::GaussParams2 gp2 = pfd::make_params2(gp);
-    pfd::f32x2 nx = 0ull, ny = 0ull;  // +0.0f in both halves
-    float pxa = 0.f, pya = 0.f, pxc = 0.f, pyc = 0.f;
-    if constexpr (MODE == P2P_FAR) {
-        const float axc = (ta.x - cx) + ta.z, ayc = (ta.y - cy) + ta.w;
-        const pfd::f32x2 txc = pfd::pack2(axc, (tb.x - cx) + tb.z);
-        const pfd::f32x2 tyc = pfd::pack2(ayc, (tb.y - cy) + tb.w);
-        auto one = [&](int k) {
-            const ulonglong2 loc = lds_u64x2(a_hi + 16 * k);
-            const unsigned long long g2 = lds_u64(a_g + 8 * k);
-            if (NT >= 2)
-                pfd::pair2_far_local(loc, g2, txc, tyc, gp2, nx, ny);
-            else
-                far_local_scalar(loc, g2, axc, ayc, pxa, pya);
-        };
-        if (cnt == 32) {
-#pragma unroll(P2P_UNROLL)
-            for (int k = 0; k < 32; ++k) one(k);
-        } else {
-#pragma unroll 1
-            for (int k = 0; k < cnt; ++k) one(k);
-        }
-    } else {
-        const pfd::f32x2 txh = pfd::pack2(ta.x, tb.x), tyh = pfd::pack2(ta.y, tb.y);
-        const pfd::f32x2 txl = pfd::pack2(ta.z, tb.z), tyl = pfd::pack2(ta.w, tb.w);
-        if (cnt == 32) {  // full chunk (the common case)
-#pragma unroll(P2P_UNROLL)
-            for (int k = 0; k < 32; ++k)
-                p2p_pair<NT, MODE>(lds_u64x2(a_hi + 16 * k), lds_u64x2(a_lo + 16 * k),
-                                   lds_u64(a_g + 8 * k), txh, tyh, txl, tyl, ta, tc, gp, gp2, nx,
-                                   ny, pxa, pya, pxc, pyc);
-        } else {  // the rest of a buffer at the end of a group: kept small in code
-#pragma unroll 1
-            for (int k = 0; k < cnt; ++k)
-                p2p_pair<NT, MODE>(lds_u64x2(a_hi + 16 * k), lds_u64x2(a_lo + 16 * k),
-                                   lds_u64(a_g + 8 * k), txh, tyh, txl, tyl, ta, tc, gp, gp2, nx,
-                                   ny, pxa, pya, pxc, pyc);
-        }
-    }
-    P2PSums r;
-    if (NT >= 2) {
-        float nxa, nxb, nya, nyb;
-        pfd::unpack2(nx, nxa, nxb);
-        pfd::unpack2(ny, nya, nyb);
-        r.s[0] = -nxa;
-        r.s[1] = nya;
-        r.s[2] = -nxb;
-        r.s[3] = nyb;
-    } else {
-        r.s[0] = pxa;
-        r.s[1] = pya;
-        r.s[2] = r.s[3] = 0.f;
-    }
-    r.s[4] = pxc;
-    r.s[5] = pyc;
-    return r;
-}
-
-template <int NT, int MODE>
-__device__ __forceinline__ void p2p_chunk(const ulonglong2 *shi, const ulonglong2 *slo,
-                                          const unsigned long long *sg2, int cnt,
-                                          const float4 &ta, const float4 &tb, const float4 &tc,
-                                          float cx, float cy, const pfd::GaussParams &gp,
-                                          float (&acc)[16]) {
-    const P2PSums r = p2p_chunk_sums<NT, MODE>(
-        (uint32_t)__cvta_generic_to_shared(shi), (uint32_t)__cvta_generic_to_shared(slo),
-        (uint32_t)__cvta_generic_to_shared(sg2), cnt, ta, tb, tc, cx, cy, gp);
-    pfd::comp_add(acc[0], acc[1], r.s[0]);
-    pfd::comp_add(acc[2], acc[3], r.s[1]);
-    if (NT >= 2) {
-        pfd::comp_add(acc[4], acc[5], r.s[2]);
-        pfd::comp_add(acc[6], acc[7], r.s[3]);
-    }
-    if (NT == 3) {
-        pfd::comp_add(acc[8], acc[9], r.s[4]);
-        pfd::comp_add(acc[10], acc[11], r.s[5]);
-    }
-}
-
-// The third target slot of a group of 65..96 targets: the rem = size - 64
-// remainder targets are paired (c, d) into rp = ceil(rem / 2) packed pairs
-// spread over the warp, m = 32 / rp lanes per pair, lane (j + rp q) taking
-// sources q, q + m, q + 2m, ... of the chunk for pair j with the packed pair
-// code of the main slots; the m partial sums are combined at the end of the
-// group.  Lanes with no share get q >= 32.  Returns -nx_c, ny_c, -nx_d, ny_d.
-template <int MODE>
-__device__ __noinline__ float4 p2p_split_sums(uint32_t a_hi, uint32_t a_lo, uint32_t a_g, int cnt,
-                                              int q, int m, float4 tc, float4 td, float cx,
-                                              float cy, pfd::GaussParams gp) {
-    const pfd::GaussParams2 gp2 = pfd::make_params2(gp);
-    pfd::f32x2 nx = 0ull, ny = 0ull;
-    if constexpr (MODE == P2P_FAR) {
-        const pfd::f32x2 txc = pfd::pack2((tc.x - cx) + tc.z, (td.x - cx) + td.z);
-        const pfd::f32x2 tyc = pfd::pack2((tc.y - cy) + tc.w, (td.y - cy) + td.w);
-#pragma unroll 2
-        for (int k = q; k < cnt; k += m)
-            pfd::pair2_far_local(lds_u64x2(a_hi + 16 * k), lds_u64(a_g + 8 * k), txc, tyc, gp2, nx,
-                                 ny);
-    } else {
-        const pfd::f32x2 txh = pfd::pack2(tc.x, td.x), tyh = pfd::pack2(tc.y, td.y);
-        const pfd::f32x2 txl = pfd::pack2(tc.z, td.z), tyl = pfd::pack2(tc.w, td.w);
-#pragma unroll 2
-        for (int k = q; k < cnt; k += m)
-            pfd::pair2<MODE == P2P_SERIES>(lds_u64x2(a_hi + 16 * k), lds_u64x2(a_lo + 16 * k),
-                                            lds_u64(a_g + 8 * k), txh, tyh, txl, tyl, gp2, nx, ny);
-    }
-    float nxc, nxd, nyc, nyd;
-    pfd::unpack2(nx, nxc, nxd);
-    pfd::unpack2(ny, nyc, nyd);
-    return make_float4(-nxc, nyc, -nxd, nyd);
-}
-
-// p2p_chunk for the group's targets-per-lane count nt (warp-uniform).
-// nt = 3: targets a, b packed plus the lane's share (qs of msp) of a
-// remainder target pair (c, d).
-template <int MODE>
-__device__ __forceinline__ void p2p_run_chunk(int nt, const ulonglong2 *shi, const ulonglong2 *slo,
-                                              const unsigned long long *sg2, int cnt,
-                                              const float4 &ta, const float4 &tb,
-                                              const float4 &tc, const float4 &td, int qs,
-                                              int msp, float cx, float cy,
-                                              const pfd::GaussParams &gp, float (&acc)[16]) {
-    if (nt == 1) {
-        p2p_chunk<1, MODE>(shi, slo, sg2, cnt, ta, tb, tc, cx, cy, gp, acc);
-        return;
-    }
-    p2p_chunk<2, MODE>(shi, slo, sg2, cnt, ta, tb, tc, cx, cy, gp, acc);
-    if (nt == 3) {
-        const float4 r = p2p_split_sums<MODE>(
-            (uint32_t)__cvta_generic_to_shared(shi), (uint32_t)__cvta_generic_to_shared(slo),
-            (uint32_t)__cvta_generic_to_shared(sg2), cnt, qs, msp, tc, td, cx, cy, gp);
-        pfd::comp_add(acc[8], acc[9], r.x);
-        pfd::comp_add(acc[10], acc[11], r.y);
-        pfd::comp_add(acc[12], acc[13], r.z);
-        pfd::comp_add(acc[14], acc[15], r.w);
-    }
-}
-
-__device__ __forceinline__ float warp_min(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fminf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
-__device__ __forceinline__ float warp_max(float v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
-constexpr int P2P_OWN_GROUPS = 4;  // target groups a block's own CTA computes at most
-
-
-// Target group gi of block b (groups of at most 96 targets, balanced: sizes
-// differ by at most one; every group streams all the block's sources, so a
-// small last group would cost nearly as much as a full one) against the
-// block's whole source stream; writes the group's near-field velocities.
-__device__ __forceinline__ void p2p_group_body(
-    int64_t b, int t0, int tn, int ngrp, int gi, const int32_t *__restrict__ sstart,
-    const int32_t *__restrict__ scnt, const float4 *__restrict__ shl,
-    const float *__restrict__ sg32, const float4 *__restrict__ thl,
-    const int32_t *__restrict__ run_off, const int2 *__restrict__ runs, pfd::GaussParams gp,
-    double2 *__restrict__ nearv, ulonglong2 (*s_hi)[P2P_BUF], ulonglong2 (*s_lo)[P2P_BUF],
-    unsigned long long (*s_g2)[P2P_BUF], int *s_rs, int *s_rp, unsigned long long &npairs,
-    unsigned long long &nfar, int64_t ns_all, int64_t nt_all) {
-    const int lane = threadIdx.x;
-    const unsigned lt = (1u << lane) - 1u;
-    const float rser = sqrtf(gp.r2_series);
-    const int r0 = run_off[b], r1 = run_off[b + 1];
-    const int tg = (int)((int64_t)gi * tn / ngrp);
-    const int gsz = (int)((int64_t)(gi + 1) * tn / ngrp) - tg;
-    const int nt = (gsz <= 32) ? 1 : (gsz <= 64) ? 2 : 3;  // warp-uniform
-    // nt = 3: remainder targets tg + 64 + j, j < rem, in rp packed pairs
-    // (tg + 64 + 2 p, + 1), each pair on msp lanes
-    const int rem = nt == 3 ? gsz - 64 : 32;
-    const int rp = (rem + 1) / 2;
-    const int msp = 32 / rp;
-    const bool cval = nt == 3 && lane < rp * msp;
-    const int qs = cval ? lane / rp : 32;
-    const int ia = tg + lane, ib = tg + 32 + lane, ic = tg + 64 + 2 * (lane % rp), id = ic + 1;
-    const bool dval = cval && id < tg + gsz;
-    const float4 z4 = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (!PF_IDX_OK((int64_t)t0 + tg + gsz - 1, nt_all, 204)) return;  // the group's last target
-    const float4 ta = (lane < gsz) ? thl[t0 + ia] : z4;
-    const float4 tb = (lane + 32 < gsz) ? thl[t0 + ib] : z4;
-    const float4 tc = cval ? thl[t0 + ic] : z4;
-    const float4 td = dval ? thl[t0 + id] : tc;  // an odd remainder's last pair repeats c
-    // box of the group's targets (hi parts), for the series-free test
-    float bx0 = INFINITY, bx1 = -INFINITY, by0 = INFINITY, by1 = -INFINITY;
-    if (lane < gsz) { bx0 = bx1 = ta.x; by0 = by1 = ta.y; }
-    if (lane + 32 < gsz) { bx0 = fminf(bx0, tb.x); bx1 = fmaxf(bx1, tb.x); by0 = fminf(by0, tb.y); by1 = fmaxf(by1, tb.y); }
-    if (cval) { bx0 = fminf(bx0, fminf(tc.x, td.x)); bx1 = fmaxf(bx1, fmaxf(tc.x, td.x)); by0 = fminf(by0, fminf(tc.y, td.y)); by1 = fmaxf(by1, fmaxf(tc.y, td.y)); }
-    bx0 = warp_min(bx0);
-    bx1 = warp_max(bx1);
-    by0 = warp_min(by0);
-    by1 = warp_max(by1);
-    // a source at box distance d has r2 >= (d - e)^2 for every target, e
-    // covering the hi-part rounding of both points (2^-23 relative each)
-    const float mag = fmaxf(fmaxf(fabsf(bx0), fabsf(bx1)), fmaxf(fabsf(by0), fabsf(by1)));
-    const float reach = rser * 1.001f + (mag + rser) * 4.8e-7f + 1e-30f;
-    const float reach2 = reach * reach;
-    const float rfar = sqrtf(gp.r2_far);
-    const float reachf = rfar * 1.001f + (mag + rfar) * 4.8e-7f + 1e-30f;
-    const float reachf2 = reachf * reachf;
-    // centre for the far sources' relative coordinates (any float near the group)
-    const float cx = 0.5f * (bx0 + bx1), cy = 0.5f * (by0 + by1);
-    float acc[16] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f,
-                     0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-    // the three buffers are rings of P2P_BUF = 64 entries: entries waiting
-    // c0, c1, c2 from heads h0, h1, h2; a chunk is always the 32 entries at
-    // the head (0 or 32), so it never wraps, and taking it flips the head
-    int c0 = 0, c1 = 0, c2 = 0;
-    int h0 = 0, h1 = 0, h2 = 0;
-    for (int rc = r0; rc < r1; rc += P2P_RUNS_SM) {
-        const int nrc = min(P2P_RUNS_SM, r1 - rc);
-        int pre = 0;
-        for (int k0 = 0; k0 < nrc; k0 += 32) {
-            const int k = k0 + lane;
-            int st = 0, len = 0;
-            if (k < nrc) {
-                const int2 rr = runs[rc + k];
-                st = sstart[rr.x];
-                len = sstart[rr.y] + scnt[rr.y] - st;
-            }
-            int inc = len;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += t;
-            }
-            if (k < nrc) {
-                s_rs[k] = st;
-                s_rp[k] = pre + inc - len;
-            }
-            pre += __shfl_sync(0xffffffffu, inc, 31);
-        }
-        if (lane == 0) s_rp[nrc] = pre;
-        __syncwarp();
-        const int S = pre;
-        npairs += (unsigned long long)S * (unsigned long long)gsz;
-        // each lane's stream position only moves forward (by 32 per
-        // round), so the run holding it is found by advancing an index:
-        // the largest r with prefix[r] <= p (empty runs are stepped over).
-        // The loads of round s0 + 32 are issued before round s0's chunks
-        // run, so their latency overlaps the pair work.
-        int rr = 0;
-        float4 spv = z4;
-        float gg = 0.f;
-        auto fetch = [&](int p, float4 &v, float &w) {
-            if (p < S) {
-                while (rr + 1 < nrc && s_rp[rr + 1] <= p) ++rr;
-                const int src = s_rs[rr] + (p - s_rp[rr]);
-                if (PF_IDX_OK(src, ns_all, 203)) {
-                    v = shl[src];
-                    w = sg32[src];
-                }
-            }
-        };
-        fetch(lane, spv, gg);
-        for (int s0 = 0; s0 < S; s0 += 32) {
-            const int p = s0 + lane;
-            int cls = -1;  // 0 far, 1 full, 2 series; -1 past the stream
-            if (p < S) {
-                const float ex = fmaxf(fmaxf(bx0 - spv.x, spv.x - bx1), 0.f);
-                const float ey = fmaxf(fmaxf(by0 - spv.y, spv.y - by1), 0.f);
-                const float d2 = ex * ex + ey * ey;
-                cls = d2 > reachf2 ? 0 : d2 > reach2 ? 1 : 2;
-            }
-            // append each source to the buffer of its mode, in stream order
-            const unsigned m0 = __ballot_sync(0xffffffffu, cls == 0);
-            const unsigned m1 = __ballot_sync(0xffffffffu, cls == 1);
-            const unsigned m2 = __ballot_sync(0xffffffffu, cls == 2);
-            if (cls >= 0) {
-                const unsigned mm = cls == 0 ? m0 : cls == 1 ? m1 : m2;
-                const int k =
-                    ((cls == 0 ? h0 + c0 : cls == 1 ? h1 + c1 : h2 + c2) + __popc(mm & lt)) &
-                    (P2P_BUF - 1);
-                if (cls == 0) {  // far: coordinates relative to the group centre
-                    const float lx = (spv.x - cx) + spv.z, ly = (spv.y - cy) + spv.w;
-                    s_hi[0][k] = make_ulonglong2(pfd::pack2(lx, lx), pfd::pack2(ly, ly));
-                } else {
-                    s_hi[cls][k] = make_ulonglong2(pfd::pack2(spv.x, spv.x),
-                                                   pfd::pack2(spv.y, spv.y));
-                    s_lo[cls][k] = make_ulonglong2(pfd::pack2(spv.z, spv.z),
-                                                   pfd::pack2(spv.w, spv.w));
-                }
-                s_g2[cls][k] = pfd::pack2(gg, gg);
-            }
-            c0 += __popc(m0);
-            c1 += __popc(m1);
-            c2 += __popc(m2);
-            spv = z4;
-            gg = 0.f;
-            fetch(p + 32, spv, gg);
-            __syncwarp();
-            bool ran = false;  // warp-uniform
-            if (c0 >= 32) {
-                p2p_run_chunk<P2P_FAR>(nt, s_hi[0] + h0, s_lo[0] + h0, s_g2[0] + h0, 32, ta, tb,
-                                       tc, td, qs, msp, cx, cy, gp, acc);
-                nfar += 32ull * (unsigned long long)gsz;
-                c0 -= 32;
-                h0 ^= 32;
-                ran = true;
-            }
-            if (c1 >= 32) {
-                p2p_run_chunk<P2P_FULL>(nt, s_hi[1] + h1, s_lo[1] + h1, s_g2[1] + h1, 32, ta,
-                                        tb, tc, td, qs, msp, cx, cy, gp, acc);
-                c1 -= 32;
-                h1 ^= 32;
-                ran = true;
-            }
-            if (c2 >= 32) {
-                p2p_run_chunk<P2P_SERIES>(nt, s_hi[2] + h2, s_lo[2] + h2, s_g2[2] + h2, 32, ta,
-                                          tb, tc, td, qs, msp, cx, cy, gp, acc);
-                c2 -= 32;
-                h2 ^= 32;
-                ran = true;
-            }
-            if (ran) __syncwarp();  // the chunks are read before the next round refills them
-        }
-    }
-    // what is left in the buffers (fewer than 32 each)
-    // (fewer than 32 from a head of 0 or 32: no wrap)
-    if (c0)
-        p2p_run_chunk<P2P_FAR>(nt, s_hi[0] + h0, s_lo[0] + h0, s_g2[0] + h0, c0, ta, tb, tc,
-                               td, qs, msp, cx, cy, gp, acc);
-    nfar += (unsigned long long)c0 * (unsigned long long)gsz;
-    if (c1)
-        p2p_run_chunk<P2P_FULL>(nt, s_hi[1] + h1, s_lo[1] + h1, s_g2[1] + h1, c1, ta, tb, tc,
-                                td, qs, msp, cx, cy, gp, acc);
-    if (c2)
-        p2p_run_chunk<P2P_SERIES>(nt, s_hi[2] + h2, s_lo[2] + h2, s_g2[2] + h2, c2, ta, tb,
-                                  tc, td, qs, msp, cx, cy, gp, acc);
-    __syncwarp();
-    if (lane < gsz)
-        nearv[t0 + ia] = make_double2(INV_2PI * ((double)acc[0] + (double)acc[1]),
-                                      INV_2PI * ((double)acc[2] + (double)acc[3]));
-    if (lane + 32 < gsz)
-        nearv[t0 + ib] = make_double2(INV_2PI * ((double)acc[4] + (double)acc[5]),
-                                      INV_2PI * ((double)acc[6] + (double)acc[7]));
-    if (nt == 3) {  // combine the msp shares of each remainder pair, in lane order
-        float h[4] = {acc[8], acc[10], acc[12], acc[14]};
-        float l[4] = {acc[9], acc[11], acc[13], acc[15]};
-        for (int q = 1; q < msp; ++q) {
-            const int sl = lane % rp + rp * q;  // < rp * msp <= 32
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                const float a = __shfl_sync(0xffffffffu, acc[8 + 2 * v], sl);
-                const float b = __shfl_sync(0xffffffffu, acc[9 + 2 * v], sl);
-                pfd::comp_add(h[v], l[v], a);
-                l[v] += b;
-            }
-        }
-        if (lane < rp) {
-            nearv[t0 + ic] = make_double2(INV_2PI * ((double)h[0] + (double)l[0]),
-                                          INV_2PI * ((double)h[1] + (double)l[1]));
-            if (dval)
-                nearv[t0 + id] = make_double2(INV_2PI * ((double)h[2] + (double)l[2]),
-                                              INV_2PI * ((double)h[3] + (double)l[3]));
-        }
-    }
-}
-
-// Shared memory of one P2P CTA (one warp).
-struct P2PSmem {
-    // source buffers, one per mode: [P2P_FAR], [P2P_FULL], [P2P_SERIES]
-    ulonglong2 hi[3][P2P_BUF];  // {x_hi, x_hi}, {y_hi, y_hi}
-    ulonglong2 lo[3][P2P_BUF];  // {x_lo, x_lo}, {y_lo, y_lo}
-    unsigned long long g2[3][P2P_BUF];  // {g, g}
-    int rs[P2P_RUNS_SM];      // particle start of run
-    int rp[P2P_RUNS_SM + 1];  // stream prefix of run
-};
-
-// Targets of P2P block b: first sorted target t0, count returned.
-__device__ __forceinline__ int p2p_targets(const P2PDesc &d, int64_t b, int &t0) {
-    const uint32_t leaf0 = (uint32_t)b << (2 * d.kb), nl = 1u << (2 * d.kb);
-    t0 = d.tstart[leaf0];
-    return d.tstart[leaf0 + nl - 1] + d.tcnt[leaf0 + nl - 1] - t0;
-}
-
-__device__ __forceinline__ void p2p_group(const P2PDesc &d, int64_t b, int t0, int tn, int ngrp,
-                                          int gi, P2PSmem &sm, unsigned long long &npairs,
-                                          unsigned long long &nfar) {
-    p2p_group_body(b, t0, tn, ngrp, gi, d.sstart, d.scnt, d.shl, d.sg32, d.thl, d.run_off, d.runs,
-                   d.gp, d.nearv, sm.hi, sm.lo, sm.g2, sm.rs, sm.rp, npairs, nfar, d.work.ns,
-                   d.work.nt);
-}
-
-// The CTA of P2P block `local` (launch order): its target groups, unless
-// there are more than P2P_OWN_GROUPS of them: such a block (a dense cluster)
-// is listed as heavy for the second launch.
-__device__ __forceinline__ void p2p_own_block(const P2PDesc &d, int64_t local, P2PSmem &sm,
-                                              unsigned long long &npairs,
-                                              unsigned long long &nfar) {
-    const int64_t b = d.order[local];
+// The target groups beyond a block's first, as (block, group): their CTAs run
+// beside the first groups' instead of after them in one CTA (1.8e6 blobs in an
+// annulus, three groups in each occupied block: P2P 2.34 -> 2.02 ms).  Each
+// group is computed by one CTA, so results do not depend on the list's order.
+__global__ void __launch_bounds__(256) k_p2p_more_groups(const P2PDesc d) {
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= d.nblk) return;
+    const int b = d.order[i];
     int t0;
-    const int tn = p2p_targets(d, b, t0);
-    if (tn == 0) return;
-    const int ngrp = (tn + 95) / 96;
-    if (ngrp > P2P_OWN_GROUPS) {  // left to the second launch
-        if (threadIdx.x == 0) d.work.heavy[atomicAdd(d.work.heavy_n, 1u)] = (int32_t)b;
-    } else {
-        for (int gi = 0; gi < ngrp; ++gi) p2p_group(d, b, t0, tn, ngrp, gi, sm, npairs, nfar);
-    }
+    const int ngrp = p2p_groups(p2p_targets(d, b, t0));
+    if (ngrp < 2) return;
+    const int64_t at = atomicAdd(d.nmore, (unsigned)(ngrp - 1));
+    for (int g = 1; g < ngrp; ++g)
+        if (PF_IDX_OK(at + g - 1, d.more_cap, 207)) d.more[at + g - 1] = make_int2(b, g);
 }
 
-// The groups of one heavy block, shared out through its counter (counters
-// only, no waits; each group is computed by exactly one CTA, so results do
-// not depend on the schedule).
-__device__ __forceinline__ void p2p_heavy_block(const P2PDesc &d, int64_t b, P2PSmem &sm,
-                                                unsigned long long &npairs,
-                                                unsigned long long &nfar) {
-    int t0;
-    const int tn = p2p_targets(d, b, t0);
-    const int ngrp = (tn + 95) / 96;
-    for (;;) {
-        unsigned gi = 0;
-        if (threadIdx.x == 0) gi = atomicAdd((unsigned *)&d.work.grp_next[b], 1u);
-        gi = __shfl_sync(0xffffffffu, gi, 0);
-        if ((int)gi >= ngrp) break;
-        p2p_group(d, b, t0, tn, ngrp, (int)gi, sm, npairs, nfar);
-    }
-}
-
-__device__ __forceinline__ void p2p_heavy_blocks(const P2PDesc &d, P2PSmem &sm,
-                                                 unsigned long long &npairs,
-                                                 unsigned long long &nfar) {
-    const unsigned nh = *d.work.heavy_n;  // complete: written by the first launch
-    for (unsigned k = 0; k < nh; ++k) p2p_heavy_block(d, d.work.heavy[k], sm, npairs, nfar);
-}
-
-__device__ __forceinline__ void p2p_count(const P2PDesc &d, unsigned long long npairs,
-                                          unsigned long long nfar) {
-    if (threadIdx.x == 0 && (npairs | nfar)) {
-        atomicAdd(d.pairs, npairs);
-        atomicAdd(d.pairs + 2, nfar);
-    }
-}
-
-// Two launches of one kernel.  HEAVY = false: one CTA per P2P block (in
-// launch order) computes the block's target groups (or lists the block as
-// heavy).  HEAVY = true: persistent CTAs share out the groups of the heavy
-// blocks.  Without dense clusters the second launch finds nothing to do.
-template <bool HEAVY>
+// One CTA (one warp) per target group: CTA i < nblk the first group of block i
+// of the launch order (heaviest first), the CTAs after those the other groups
+// (several each where clusters make more of them than CTAs).
 __global__ void __launch_bounds__(32, P2P_MIN_CTAS) k_p2p(const P2PDesc d) {
     __shared__ P2PSmem sm;
-    unsigned long long npairs = 0, nfar = 0;
-    if (!HEAVY) {
-        if ((int64_t)blockIdx.x >= d.nblk) return;
-        p2p_own_block(d, blockIdx.x, sm, npairs, nfar);
-    } else {
-        p2p_heavy_blocks(d, sm, npairs, nfar);
+    const unsigned nblk = (unsigned)d.nblk;
+#pragma unroll 1
+    for (unsigned t = blockIdx.x;; t += gridDim.x - nblk) {
+        int b, gi;
+        if (!p2p_task(d, t, b, gi)) return;
+        int t0;
+        const int tn = p2p_targets(d, b, t0);
+        if (tn == 0) return;
+        p2p_group(d, b, t0, tn, gi, sm);
+        if (t < nblk) return;
     }
-    p2p_count(d, npairs, nfar);
-}
-
-// SMs of the current device (cached per device; host threads may race to
-// fill an entry, all with the same value).
-static int p2p_sm_count() {
-    static std::atomic<int> cached[64];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    int v = cached[dev].load(std::memory_order_relaxed);
-    if (v == 0) {
-        if (cudaDeviceGetAttribute(&v, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || v <= 0)
-            v = 148;
-        cached[dev].store(v, std::memory_order_relaxed);
-    }
-    return v;
 }
 
 // L2P + near + scatter to input order: one thread per sorted target
@@ -1627,7 +1080,27 @@ struct FmmArgs {
     double ksigmasqr, cutoff, tol;
     int ndirect;
     double *vx, *vy;
+    int64_t nt_beside = 0;  // targets of other sets whose calls run beside this one
 };
+
+// Warps per target group (the result is the same), from the number of groups to
+// expect, this set's and those of the sets beside it in a batch: the device
+// holds 2960 one-warp CTAs (20 per SM), and one group alone is a serial chain of
+// 40-100 chunks; several warps cost barriers and exchanges, 40-75% where the
+// device is full.  P2P time with 1 / 4 / 8 warps, uniform sets: 3,001 blobs 73 /
+// 42 / 30 us; 30,000 163 / 89 / 79; 38,000 87 / 81 / 93; 100,000 185 / 163 / 187;
+// 140,000 230 / 234 / 273; 150,000 198 / 280 / 325.
+static int p2p_warps(int64_t nblk, int64_t nt, int64_t nt_beside) {
+    const int64_t groups = std::min<int64_t>(nblk + nt / P2P_GROUP, nt / 40) + nt_beside / 60;
+    return groups <= 600 ? 8 : groups <= 2200 ? 4 : 1;
+}
+
+// CTAs for the groups beyond the blocks' first: those of a layer around a body,
+// or what the device holds (mostly idle CTAs for every group there could be
+// cost 13 us at 2^20 uniform blobs).
+static int64_t p2p_more_ctas(int64_t nblk, int64_t nt, int64_t more_cap) {
+    return std::min<int64_t>(more_cap, std::max<int64_t>(148 * P2P_MIN_CTAS, nt / 60 - nblk));
+}
 
 static size_t fmm_scratch_bytes(const FmmCache &c, int64_t ns, int64_t nt, bool same) {
     const int L = c.L, NP = c.np;
@@ -1648,7 +1121,7 @@ static size_t fmm_scratch_bytes(const FmmCache &c, int64_t ns, int64_t nt, bool 
     add(16 * (size_t)nbox * NP); add(16 * (size_t)nbox * NP);  // M, L
     add(16 * nt);                                   // near velocities
     add(4 * (std::max(ns, nt) / (LEAF_SMALL + 1) + 3));  // leaves for the segment sort
-    add(4 * (64 + 2 * ((size_t)1 << (2 * (c.L - c.kb)))));  // P2P work distribution
+    add(8 * (size_t)(nt / P2P_GROUP + 1));          // P2P groups beyond the first
     add(4 * pf::scan_tmp_ints(nleaf));
     return need + 4096;
 }
@@ -1697,10 +1170,9 @@ static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, dou
     double2 *nearv = (double2 *)take(16 * nt);
     // leaves listed for the segment sort: [0] count, [1 ..] leaf ids
     int32_t *big = (int32_t *)take(4 * (std::max(ns, nt) / (LEAF_SMALL + 1) + 3));
-    // P2P work distribution: counters (64 words), heavy list, group counters
-    const int64_t nblk_w = (int64_t)1 << (2 * (L - kb));
-    const size_t p2pw_bytes = 4 * (64 + 2 * (size_t)nblk_w);
-    unsigned *p2pw_mem = (unsigned *)take(p2pw_bytes);
+    // P2P groups beyond each block's first
+    const int64_t more_cap = nt / P2P_GROUP + 1;
+    int2 *more = (int2 *)take(8 * (size_t)more_cap);
     int32_t *tmp = (int32_t *)take(4 * pf::scan_tmp_ints(nleaf));
     if (!tmp) {
         pf::set_error("pf_velocity_fmm: scratch layout error");
@@ -1749,8 +1221,11 @@ static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, dou
     pd.gp = pfd::make_gauss_params(a.ksigmasqr);
     pd.nearv = nearv;
     pd.pairs = ctr;
-    pd.work = P2PWork{p2pw_mem, (int32_t *)(p2pw_mem + 64), (int32_t *)(p2pw_mem + 64) + nblk, ns,
-                      nt};
+    pd.nmore = reinterpret_cast<unsigned *>(ctr + pf::fmmx::FMM_COUNTERS - 1);
+    pd.more = more;
+    pd.more_cap = more_cap;
+    pd.ns = ns;
+    pd.nt = nt;
 
     PF_TRY(mark(1));
     // upward pass
@@ -1799,13 +1274,15 @@ static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, dou
     PF_TRY(mark(4));
     // near field
     {
-        PF_CUDA_TRY(cudaMemsetAsync(p2pw_mem, 0, p2pw_bytes, st));
-        k_p2p<false><<<(unsigned)nblk, 32, 0, st>>>(pd);
-        PF_TRY(pf::launch_status("k_p2p"));
-        // the remaining groups of blocks with more than 96 targets (if any)
-        const int64_t grid = std::min<int64_t>((int64_t)p2p_sm_count() * P2P_MIN_CTAS, nt / 96 + 1);
-        k_p2p<true><<<(unsigned)grid, 32, 0, st>>>(pd);
-        PF_TRY(pf::launch_status("k_p2p"));
+        k_p2p_more_groups<<<(unsigned)pf::ceil_div(nblk, 256), 256, 0, st>>>(pd);
+        PF_TRY(pf::launch_status("k_p2p_more_groups"));
+        const int warps = p2p_warps(nblk, nt, a.nt_beside);
+        if (warps > 1) {
+            PF_TRY(pf::fmmx::launch_p2p_multi(pd, warps, (unsigned)(nblk + more_cap), st));
+        } else {
+            k_p2p<<<(unsigned)(nblk + p2p_more_ctas(nblk, nt, more_cap)), 32, 0, st>>>(pd);
+            PF_TRY(pf::launch_status("k_p2p"));
+        }
     }
     PF_TRY(mark(5));
     k_l2p<NP><<<(unsigned)pf::ceil_div(nt, 256), 256, 0, st>>>(nt, L, x0, y0, wl, T.x, T.y,
@@ -2167,9 +1644,9 @@ size_t plan_scratch(const Plan *p, int64_t ns, int64_t nt, bool same) {
 
 pf_status plan_exec(const Plan *p, Bump &sc, int64_t ns, const double *x, const double *y,
                     const double *g, int64_t nt, const double *xt, const double *yt,
-                    double ksigmasqr, double *vx, double *vy, unsigned long long *ctr,
-                    cudaEvent_t *ev, cudaStream_t st) {
-    FmmArgs a{ns, nt, x, y, g, xt, yt, ksigmasqr, 0.0, 0.0, 0, vx, vy};
+                    double ksigmasqr, double *vx, double *vy, int64_t nt_beside,
+                    unsigned long long *ctr, cudaEvent_t *ev, cudaStream_t st) {
+    FmmArgs a{ns, nt, x, y, g, xt, yt, ksigmasqr, 0.0, 0.0, 0, vx, vy, nt_beside};
     return fmm_exec(p->c, p->x0, p->y0, p->w0, sc, a, ctr, ev, st);
 }
 

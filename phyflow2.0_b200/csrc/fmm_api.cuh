@@ -22,8 +22,8 @@ int plan_level(const Plan *p);
 size_t plan_scratch(const Plan *p, int64_t ns, int64_t nt, bool same);
 pf_status plan_exec(const Plan *p, Bump &sc, int64_t ns, const double *x, const double *y,
                     const double *g, int64_t nt, const double *xt, const double *yt,
-                    double ksigmasqr, double *vx, double *vy, unsigned long long *ctr,
-                    cudaEvent_t *ev, cudaStream_t st);
+                    double ksigmasqr, double *vx, double *vy, int64_t nt_beside,
+                    unsigned long long *ctr, cudaEvent_t *ev, cudaStream_t st);
 // leaf level from the blob count, as the reference's level count
 int auto_level(int64_t ns, int ndirect);
 // expansion terms for a tolerance
@@ -32,17 +32,9 @@ int np_for_tol(double tol);
 void tuning_get(int *leaf_level, int *np, int *kb);
 void tuning_set(int leaf_level, int np, int kb);
 constexpr int MAX_LEVEL = 11;
-// device counters one FMM call writes (see exec_fmm)
-constexpr int FMM_COUNTERS = 3;
-
-// Work-distribution state of the P2P launches of one FMM call, zeroed before
-// the first.
-struct P2PWork {
-    unsigned *heavy_n;   // entries in heavy
-    int32_t *heavy;      // blocks with several target groups [nblk]
-    int32_t *grp_next;   // groups of each heavy block handed out so far [nblk]
-    int64_t ns, nt;      // sorted sources and targets (bounds-checked build)
-};
+// device counters one FMM call writes (see exec_fmm); the last counts the
+// P2P groups beyond each block's first
+constexpr int FMM_COUNTERS = 4;
 
 // Everything the near field (P2P) of one FMM call reads and writes: its
 // sorted points and leaf tables, the plan's run lists and launch order, the
@@ -60,8 +52,14 @@ struct P2PDesc {
     pfd::GaussParams gp;
     double2 *nearv;
     unsigned long long *pairs;
-    P2PWork work;
+    unsigned *nmore;     // entries of more (a counter of the call, zeroed with the others)
+    int2 *more;          // (block, group) of the target groups beyond a block's first [more_cap]
+    int64_t more_cap;    // nt / 96 + 1 bounds them
+    int64_t ns, nt;      // sorted sources and targets (bounds-checked build)
 };
+
+// The near field with `warps` (4 or 8) warps per target group (p2p_multi.cu).
+pf_status launch_p2p_multi(const P2PDesc &d, int warps, unsigned grid, cudaStream_t st);
 
 }  // namespace fmmx
 }  // namespace pf

@@ -247,3 +247,27 @@ def test_leaf_sizes_around_the_segment_sort(k):
     assert np.array_equal(a[0], b[0]) and np.array_equal(a[1], b[1])
     rx, ry = oracle.velocity_direct(x, y, g, 2 * 0.004 ** 2)
     assert normwise_err(*a, rx, ry) <= TOL
+
+
+@pytest.mark.parametrize("n", [600, 2000, 23900, 31000, 112000, 114000])
+@pytest.mark.parametrize("cluster", [0, 1500])
+def test_near_field_warps_per_group(n, cluster):
+    """The near field's warps per target group change with the number of groups
+    (8, 4, 1 warps at about 600 and 2200 groups): uniform sets on both sides of
+    each, and with a cluster that makes one block hold many groups, against the
+    oracle; separate targets of an odd number too."""
+    rng = np.random.default_rng(n + cluster)
+    x, y = rng.random(n), rng.random(n)
+    k = min(cluster, n // 2)
+    x[:k], y[:k] = 0.3 + 2e-3 * rng.random(k), 0.6 + 2e-3 * rng.random(k)
+    g = rng.standard_normal(n) / n
+    sigma = 2.0 / np.sqrt(n)
+    vx, vy = fmm(x, y, g, sigma)
+    sub = np.concatenate([rng.choice(n, min(n, 1500), replace=False), np.arange(min(k, 300))])
+    rx, ry = oracle.velocity_direct(x, y, g, 2 * sigma * sigma, x[sub].copy(), y[sub].copy())
+    assert normwise_err(vx[sub], vy[sub], rx, ry) <= TOL
+    xt, yt = rng.random(n // 3 + 1), rng.random(n // 3 + 1)
+    vx, vy = fmm(x, y, g, sigma, xt=xt, yt=yt)
+    sub = rng.choice(xt.size, min(xt.size, 1000), replace=False)
+    rx, ry = oracle.velocity_direct(x, y, g, 2 * sigma * sigma, xt[sub].copy(), yt[sub].copy())
+    assert normwise_err(vx[sub], vy[sub], rx, ry) <= TOL
