@@ -576,6 +576,7 @@ k_l2l_tc(int l, bool two_level, const int32_t *__restrict__ tcnt, double2 *__res
 }
 
 constexpr int M2L_THREADS = 128;  // 4 warps, four target boxes each
+constexpr int64_t M2L_AHEAD_QUADS = 1365;  // box quads up to which k_m2l loads ahead (6 levels)
 
 // M2L for all levels 2..L on the FP64 tensor cores.  One translation adds
 //   L_n += r^(n+1) sum_k C(n+k, k) c_k,   c_k = (-1)^(k+1) M_k r^k
@@ -586,7 +587,14 @@ constexpr int M2L_THREADS = 128;  // 4 warps, four target boxes each
 // the real and imaginary parts of their c.  Per far-list entry: B from the
 // four sources' multipoles, KS mma per 8 rows, then lane (n = lane/4 + 8 mt,
 // box lane%4) scales its (re, im) pair by r^(n+1) into its coefficient.
-template <int NP>
+//
+// AHEAD (trees whose quads leave the device half empty): the next entry's
+// counts, multipoles and powers are loaded before the current entry's products,
+// so that a warp's chain is products, not load latency; the sums are the same.
+// One warp per CTA there.  M2L time without / with it: 3,001 blobs (85 quads) 34 /
+// 23 us, 60,007 (1365) 41 / 29, 150,000 (5461 quads) 58 / 66, 2^20 (21845) 135 /
+// 160: up to M2L_AHEAD_QUADS, and where no other sets run beside this one.
+template <int NP, bool AHEAD>
 __global__ void __launch_bounds__(M2L_THREADS)
 k_m2l(int L, int Bp, int64_t nquad, const int32_t *__restrict__ scnt,
       const int32_t *__restrict__ tcnt, const double2 *__restrict__ M, double2 *__restrict__ Lc,
@@ -595,7 +603,8 @@ k_m2l(int L, int Bp, int64_t nquad, const int32_t *__restrict__ scnt,
       unsigned long long *__restrict__ ntrans) {
     constexpr int MT = (NP + 7) / 8, KS = (NP + 3) / 4;
     const int lane = threadIdx.x & 31;
-    const int64_t u = (int64_t)blockIdx.x * (M2L_THREADS / 32) + (threadIdx.x >> 5);
+    constexpr int NWARP = AHEAD ? 1 : M2L_THREADS / 32;
+    const int64_t u = (int64_t)blockIdx.x * NWARP + (threadIdx.x >> 5);
     if (u >= nquad) return;  // the whole warp
     int l = 2;
     int64_t j = u;
@@ -633,8 +642,12 @@ k_m2l(int L, int Bp, int64_t nquad, const int32_t *__restrict__ scnt,
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) acc[mt] = make_double2(0.0, 0.0);
     unsigned nt = 0;
-    for (int e = 0; e < len; ++e) {
-        const int4 f = far[e0 + e];
+    // one far-list entry as the lane needs it
+    struct Entry {
+        double2 mv[KS], rv[KS], rs[MT];  // multipoles, powers, the scaling's powers
+        bool use;
+    };
+    auto fetch = [&](const int4 &f, Entry &t) {
         const int sx = ixb + f.x, sy = iyb + f.y;
         const bool inr = liveb && sx >= 0 && sy >= 0 && sx < side && sy < side;
         const int64_t sg = inr ? lo + morton_add(mb, (uint32_t)f.w) : 0;
@@ -642,23 +655,31 @@ k_m2l(int L, int Bp, int64_t nquad, const int32_t *__restrict__ scnt,
         // in range either way); an empty source is then skipped
         const int cs = inr ? scnt[sg] : 0;
         const double2 *rp = pw + (int64_t)f.z * (NP + 1);
-        double2 mv[KS], rv[KS];
 #pragma unroll
         for (int s = 0; s < KS; ++s) {
             const int k = 4 * s + kq;
-            mv[s] = (inr && k < NP) ? M[sg * NP + k] : make_double2(0.0, 0.0);
-            rv[s] = (k < NP) ? rp[k] : make_double2(0.0, 0.0);
+            t.mv[s] = (inr && k < NP) ? M[sg * NP + k] : make_double2(0.0, 0.0);
+            t.rv[s] = (k < NP) ? rp[k] : make_double2(0.0, 0.0);
         }
-        const bool use = inr && cs != 0;
-        if (!__any_sync(0xffffffffu, use)) continue;
-        const bool used = __shfl_sync(0xffffffffu, use, 8 * td);
-        nt += ((lane & 7) == 0 && use) ? 1u : 0u;
+        if (AHEAD)
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+                const int n = 8 * mt + nr;
+                t.rs[mt] = n < NP ? rp[n + 1] : make_double2(0.0, 0.0);
+            }
+        t.use = inr && cs != 0;
+    };
+    auto add = [&](const int4 &f, const Entry &t) {
+        if (!__any_sync(0xffffffffu, t.use)) return;
+        const bool used = __shfl_sync(0xffffffffu, t.use, 8 * td);
+        nt += ((lane & 7) == 0 && t.use) ? 1u : 0u;
+        const double2 *rp = pw + (int64_t)f.z * (NP + 1);
         double b[KS];
 #pragma unroll
         for (int s = 0; s < KS; ++s) {
-            const double2 m = mv[s], r = rv[s];
+            const double2 m = t.mv[s], r = t.rv[s];
             const double v = part ? fma(m.x, r.y, m.y * r.x) : fma(m.x, r.x, -(m.y * r.y));
-            b[s] = use ? sgn * v : 0.0;
+            b[s] = t.use ? sgn * v : 0.0;
         }
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt) {
@@ -666,7 +687,32 @@ k_m2l(int L, int Bp, int64_t nquad, const int32_t *__restrict__ scnt,
 #pragma unroll
             for (int s = 0; s < KS; ++s) mma_f64(d0, d1, af[mt][s], b[s]);
             const int n = 8 * mt + nr;
-            if (used && n < NP) acc[mt] = cfma(rp[n + 1], make_double2(d0, d1), acc[mt]);
+            if (used && n < NP)
+                acc[mt] = cfma(AHEAD ? t.rs[mt] : rp[n + 1], make_double2(d0, d1), acc[mt]);
+        }
+    };
+    if constexpr (AHEAD) {
+        if (len > 0) {
+            int4 f0 = far[e0], f1 = far[e0 + min(1, len - 1)];
+            Entry t0;
+            fetch(f0, t0);
+#pragma unroll 2
+            for (int e = 0; e < len; ++e) {
+                const int4 f2 = far[e0 + min(e + 2, len - 1)];
+                Entry t1;
+                fetch(f1, t1);  // past the end: the last entry again, not added
+                add(f0, t0);
+                t0 = t1;
+                f0 = f1;
+                f1 = f2;
+            }
+        }
+    } else {
+        for (int e = 0; e < len; ++e) {
+            const int4 f = far[e0 + e];
+            Entry t;
+            fetch(f, t);
+            add(f, t);
         }
     }
     if (lived) {
@@ -1251,9 +1297,14 @@ static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, dou
     const int B = 1 << kb, Bp = B > 2 ? B : 2;
     {
         const int64_t nquad = (nbox - level_off(2)) / 4;  // box quads of levels 2..L
-        k_m2l<NP><<<(unsigned)pf::ceil_div(nquad, M2L_THREADS / 32), M2L_THREADS, 0, st>>>(
-            L, Bp, nquad, scnt_all, tcnt_all, M, Lc, c.d_far, c.d_far_ptr, c.maxpos, c.d_pw,
-            c.d_bin, ctr + 1);
+        if (nquad <= M2L_AHEAD_QUADS && a.nt_beside == 0)
+            k_m2l<NP, true><<<(unsigned)nquad, 32, 0, st>>>(
+                L, Bp, nquad, scnt_all, tcnt_all, M, Lc, c.d_far, c.d_far_ptr, c.maxpos, c.d_pw,
+                c.d_bin, ctr + 1);
+        else
+            k_m2l<NP, false><<<(unsigned)pf::ceil_div(nquad, M2L_THREADS / 32), M2L_THREADS, 0,
+                               st>>>(L, Bp, nquad, scnt_all, tcnt_all, M, Lc, c.d_far,
+                                     c.d_far_ptr, c.maxpos, c.d_pw, c.d_bin, ctr + 1);
         PF_TRY(pf::launch_status("k_m2l"));
     }
     PF_TRY(mark(3));
