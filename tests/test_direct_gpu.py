@@ -120,3 +120,17 @@ def test_source_split_sizes_deterministic_vs_oracle(n):
     sub = rng.choice(n, min(n, 4096), replace=False)
     rx, ry = oracle.velocity_direct(x, y, g, 2 * sigma * sigma, x[sub].copy(), y[sub].copy())
     assert normwise_err(a[0][sub], a[1][sub], rx, ry) <= TOL
+
+
+@pytest.mark.parametrize("nt", [1, 31, 32, 33, 511, 513])
+@pytest.mark.parametrize("ns", [257, 900, 20000])
+def test_segment_reduction_edges(ns, nt):
+    """Targets around the reduction's 32-target CTAs and the tile's 512, with
+    2, 4 and up to 64 source segments, against the oracle."""
+    import pfblob
+    rng = np.random.default_rng(ns + nt)
+    x, y, g = rng.random(ns), rng.random(ns), rng.standard_normal(ns) / ns
+    xt, yt = rng.random(nt), rng.random(nt)
+    vx, vy = pfblob.velocity(x, y, g, 0.02, method=1, xEval=xt, yEval=yt)
+    rx, ry = oracle.velocity_direct(x, y, g, 2 * 0.02 ** 2, xt, yt)
+    assert normwise_err(vx, vy, rx, ry) <= TOL
