@@ -94,19 +94,38 @@ __device__ __forceinline__ void pair_velocity(const PanelSm &q, double px, doubl
     ay += q.s * vxp + q.c * vyp;
 }
 
-// One warp per group: the panels' frame records, the enclosing circle and the
-// series coefficients (lane k forms A_{k+1}).
+// base^e of a complex number by squaring (e >= 0).
+__device__ __forceinline__ double2 cpow_int(double br, double bi, int e) {
+    double pr = 1.0, pi = 0.0;
+    for (; e; e >>= 1) {
+        if (e & 1) {
+            const double t = pr * br - pi * bi;
+            pi = pr * bi + pi * br;
+            pr = t;
+        }
+        const double t = br * br - bi * bi;
+        bi = 2.0 * br * bi;
+        br = t;
+    }
+    return make_double2(pr, pi);
+}
+
+// One CTA of two warps per group: the first warp forms the panels' frame
+// records and the enclosing circle, then thread k the series coefficient
+// A_{k+1}, its powers by squaring (one multiplication after the other, up to
+// 36 of them for each of 16 panels, took 21 us for 32 groups; this takes 10).
 template <bool SOURCE, int G = PC_G>
-__global__ void __launch_bounds__(32)
+__global__ void __launch_bounds__(64)
 k_panel_groups(int64_t m, const double *__restrict__ gamma, const double *__restrict__ xs,
                const double *__restrict__ ys, const double *__restrict__ xe,
                const double *__restrict__ ye, const double *__restrict__ cosa,
                const double *__restrict__ sina, PanelGroup *__restrict__ groups,
                PanelSm *__restrict__ pan) {
     const int64_t j0 = (int64_t)blockIdx.x * G;
-    const int lane = threadIdx.x;
+    const int lane = threadIdx.x & 31;
     const int cnt = (int)min((int64_t)G, m - j0);
-    const bool has = lane < cnt;
+    const bool first = threadIdx.x < 32;
+    const bool has = first && lane < cnt;
     double x1 = 0.0, y1 = 0.0, x2e = 0.0, y2e = 0.0, kr = 0.0, ki = 0.0;
     double bx0 = INFINITY, bx1 = -INFINITY, by0 = INFINITY, by1 = -INFINITY;
     if (has) {
@@ -162,30 +181,23 @@ k_panel_groups(int64_t m, const double *__restrict__ gamma, const double *__rest
         s_e[4][lane] = kr;
         s_e[5][lane] = ki;
     }
-    __syncwarp();
+    __syncthreads();
     PanelGroup *gp = groups + blockIdx.x;
-    // terms k = lane + 1 and lane + 33 (PC_P > 32 of them)
-    for (int k = lane + 1; k <= PC_P; k += 32) {
+    const int k = threadIdx.x + 1;
+    if (k <= PC_P) {
         double sr = 0.0, si = 0.0;
+#pragma unroll 4
         for (int j = 0; j < cnt; ++j) {
-            const double jar = s_e[0][j], jai = s_e[1][j], jbr = s_e[2][j], jbi = s_e[3][j];
             const double jkr = s_e[4][j], jki = s_e[5][j];
-            double pr = 1.0, pi = 0.0, qr = 1.0, qi = 0.0;  // a^k, b^k
-            for (int e = 0; e < k; ++e) {
-                const double t1 = pr * jar - pi * jai;
-                pi = pr * jai + pi * jar;
-                pr = t1;
-                const double t2 = qr * jbr - qi * jbi;
-                qi = qr * jbi + qi * jbr;
-                qr = t2;
-            }
-            const double dr = pr - qr, di = pi - qi;
+            const double2 pa = cpow_int(s_e[0][j], s_e[1][j], k);
+            const double2 pb = cpow_int(s_e[2][j], s_e[3][j], k);
+            const double dr = pa.x - pb.x, di = pa.y - pb.y;
             sr += jkr * dr - jki * di;
             si += jkr * di + jki * dr;
         }
         gp->a[k - 1] = make_double2(sr / k, si / k);
     }
-    if (lane == 0) {
+    if (threadIdx.x == 0) {
         gp->cx = cx;
         gp->cy = cy;
         gp->R = R;
@@ -291,6 +303,7 @@ constexpr int PL_NB = 64;         // boxes per side of the grid
 constexpr int PL_P = 40;          // local expansion terms
 constexpr int64_t PL_MIN_POINTS = 32768;  // below: every group per point
 constexpr int PL_MIN_GROUPS = 8;
+constexpr int64_t PL_SLICE = (int64_t)1 << 24;  // points taken at a time
 // near groups on the box-grid path are summed by sub-groups of PL_SUB panels
 // (their own series where R_sub / |z - c_sub| <= PC_RHO, else the pair formula)
 constexpr int PL_SUB = 4;
@@ -299,6 +312,9 @@ static_assert(PC_G % PL_SUB == 0, "sub-groups tile a group");
 struct PanelGrid {
     double x0, y0, wb;  // grid origin and box width
     unsigned long long mn[2], mx[2];  // ordered images of the points' min, max
+    unsigned long long runs;          // runs of equal boxes in input order
+    int sorted;                       // points are taken in box order
+    int nocc;                         // boxes with a point
 };
 
 __device__ __forceinline__ unsigned long long pl_ord(double v) {
@@ -313,6 +329,8 @@ __device__ __forceinline__ double pl_unord(unsigned long long o) {
 __global__ void k_panel_grid_init(PanelGrid *gd) {
     gd->mn[0] = gd->mn[1] = ~0ull;
     gd->mx[0] = gd->mx[1] = 0ull;
+    gd->runs = 0ull;
+    gd->sorted = 0;
 }
 
 // min / max of the point coordinates (order-preserving integer images)
@@ -370,35 +388,144 @@ k_panel_bbox(int64_t n, const double *__restrict__ xv, const double *__restrict_
     }
 }
 
-// Boxes holding a point (the others need no local expansion); a store per
-// run of equal boxes in a warp
-__global__ void __launch_bounds__(PN_THREADS)
-k_panel_flags(int64_t n, const double *__restrict__ xv, const double *__restrict__ yv,
-              const PanelGrid *gd, int *__restrict__ flags) {
+__device__ __forceinline__ int panel_box(double px, double py, double x0, double y0, double wb) {
+    const int bx = min(max((int)floor((px - x0) / wb), 0), PL_NB - 1);
+    const int by = min(max((int)floor((py - y0) / wb), 0), PL_NB - 1);
+    return bx * PL_NB + by;
+}
+
+// Points per box; each point's box and its rank among the CTA's points of that
+// box (CTA c takes the c-th of gridDim.x equal parts of the points), and per CTA
+// the box's points of the CTAs before it in base (in the order the atomics
+// fall).  The number of runs of equal boxes in neighbouring lanes tells whether
+// the points come in an order that keeps a warp in few boxes.  (A global atomic
+// for each run took 52 us for 1.5e6 unordered points; this takes
+// 11.)
+constexpr int PCT_THREADS = 1024;
+
+__device__ __forceinline__ int64_t panel_part(int64_t n, int64_t c, int64_t parts) {
+    return min(n, c * ((n + parts - 1) / parts));
+}
+
+__global__ void __launch_bounds__(PCT_THREADS)
+k_panel_count(int64_t n, const double *__restrict__ xv, const double *__restrict__ yv,
+              PanelGrid *gd, int *__restrict__ counts, int2 *__restrict__ where,
+              int *__restrict__ base) {
+    __shared__ int s_n[PL_NB * PL_NB];
+    __shared__ int s_runs[PCT_THREADS / 32];
     const double x0 = gd->x0, y0 = gd->y0, wb = gd->wb;
     const int lane = threadIdx.x & 31;
+    for (int k = threadIdx.x; k < PL_NB * PL_NB; k += PCT_THREADS) s_n[k] = 0;
+    __syncthreads();
+    int runs = 0;
+    const int64_t lo = panel_part(n, blockIdx.x, gridDim.x);
+    const int64_t hi = panel_part(n, blockIdx.x + 1, gridDim.x);
     // four blocks of points per iteration, their loads in flight together
-    const int64_t stride = (int64_t)gridDim.x * PN_THREADS;
-    for (int64_t b0 = (int64_t)blockIdx.x * PN_THREADS; b0 < n; b0 += 4 * stride) {
+    for (int64_t b0 = lo; b0 < hi; b0 += 4 * PCT_THREADS) {
         double xs4[4], ys4[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const int64_t i = b0 + u * stride + threadIdx.x;
-            xs4[u] = i < n ? xv[i] : 0.0;
-            ys4[u] = i < n ? yv[i] : 0.0;
+            const int64_t i = b0 + u * PCT_THREADS + threadIdx.x;
+            xs4[u] = i < hi ? xv[i] : 0.0;
+            ys4[u] = i < hi ? yv[i] : 0.0;
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            const int64_t i = b0 + u * stride + threadIdx.x;
-            int box = -1;
-            if (i < n) {
-                const int bx = min(max((int)floor((xs4[u] - x0) / wb), 0), PL_NB - 1);
-                const int by = min(max((int)floor((ys4[u] - y0) / wb), 0), PL_NB - 1);
-                box = bx * PL_NB + by;
-            }
+            const int64_t i = b0 + u * PCT_THREADS + threadIdx.x;
+            const int box = i < hi ? panel_box(xs4[u], ys4[u], x0, y0, wb) : -1;
             const int prev = __shfl_up_sync(0xffffffffu, box, 1);
-            if (box >= 0 && (lane == 0 || prev != box)) flags[box] = 1;
+            const bool head = lane == 0 || prev != box;
+            const unsigned heads = __ballot_sync(0xffffffffu, head);
+            const unsigned upto = 0xffffffffu >> (31 - lane);
+            const int mine = 31 - __clz(heads & upto);  // my run's first lane
+            int first = 0;
+            if (head && box >= 0) {
+                const unsigned after = heads & ~upto;
+                first = atomicAdd(&s_n[box], (after ? __ffs(after) - 1 : 32) - lane);
+                ++runs;
+            }
+            first = __shfl_sync(0xffffffffu, first, mine);
+            if (box >= 0) where[i] = make_int2(box, first + lane - mine);
         }
+    }
+    runs = __reduce_add_sync(0xffffffffu, runs);
+    if (lane == 0) s_runs[threadIdx.x >> 5] = runs;
+    __syncthreads();
+    for (int k = threadIdx.x; k < PL_NB * PL_NB; k += PCT_THREADS)
+        if (s_n[k]) base[(int64_t)blockIdx.x * PL_NB * PL_NB + k] = atomicAdd(&counts[k], s_n[k]);
+    if (threadIdx.x == 0) {
+        for (int v = 1; v < PCT_THREADS / 32; ++v) runs += s_runs[v];
+        atomicAdd(&gd->runs, (unsigned long long)runs);
+    }
+}
+
+// First sorted position of each box (one CTA), the list of the boxes with a
+// point, and whether the points are to be
+// taken in box order: where a warp's 32 points in input order lie in more than
+// 8 boxes on average, each lane would read its own box's 40 coefficients and
+// near groups.  (1.5e6 unordered points: evaluation 319 us in input order, 99 in
+// box order after 21 for the sort; blobs in lattice order change boxes less often
+// and keep their order.)
+__global__ void __launch_bounds__(1024)
+k_panel_starts(int64_t n, PanelGrid *gd, const int *__restrict__ counts, int *__restrict__ start,
+               int *__restrict__ boxes) {
+    constexpr int PER = PL_NB * PL_NB / 1024;
+    __shared__ unsigned long long s_w[32];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    int v[PER];
+    unsigned long long sum = 0;  // points, and occupied boxes from bit 32 on
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        v[k] = counts[threadIdx.x * PER + k];
+        sum += (unsigned)v[k] + (v[k] ? 1ull << 32 : 0ull);
+    }
+    unsigned long long inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    if (lane == 31) s_w[wid] = inc;
+    __syncthreads();
+    if (wid == 0) {
+        const unsigned long long own = s_w[lane];
+        unsigned long long all = own;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long t = __shfl_up_sync(0xffffffffu, all, o);
+            if (lane >= o) all += t;
+        }
+        s_w[lane] = all - own;
+        if (lane == 31) gd->nocc = (int)(all >> 32);
+    }
+    __syncthreads();
+    unsigned long long ex = s_w[wid] + inc - sum;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) {
+        start[threadIdx.x * PER + k] = (int)(unsigned)ex;
+        if (v[k]) boxes[ex >> 32] = threadIdx.x * PER + k;
+        ex += (unsigned)v[k] + (v[k] ? 1ull << 32 : 0ull);
+    }
+    if (threadIdx.x == 0) gd->sorted = gd->runs > (unsigned long long)n / 4;
+}
+
+// The points in box order: coordinates and input index (only where k_panel_starts
+// asked for it; the same parts of the points as k_panel_count).
+__global__ void __launch_bounds__(PCT_THREADS)
+k_panel_place(int64_t n, const PanelGrid *gd, const double *__restrict__ xv,
+              const double *__restrict__ yv, const int2 *__restrict__ where,
+              const int *__restrict__ base, const int *__restrict__ start,
+              double2 *__restrict__ pts, int32_t *__restrict__ idx) {
+    if (!gd->sorted) return;
+    const int *const mine = base + (int64_t)blockIdx.x * PL_NB * PL_NB;
+    const int64_t hi = panel_part(n, blockIdx.x + 1, gridDim.x);
+#pragma unroll 4
+    for (int64_t i = panel_part(n, blockIdx.x, gridDim.x) + threadIdx.x; i < hi; i += PCT_THREADS) {
+        const int2 w = where[i];
+        const int64_t p = (int64_t)start[w.x] + mine[w.x] + w.y;
+        if (!PF_IDX_OK(p, n, 301)) continue;
+        pts[p] = make_double2(xv[i], yv[i]);
+        idx[p] = (int32_t)i;
     }
 }
 
@@ -414,125 +541,140 @@ __global__ void k_panel_grid_set(PanelGrid *gd) {
     gd->wb = e * (1.0 + 1e-9) / PL_NB;
 }
 
-// One CTA of four warps per box: the near-group mask (mwords words) and the
-// local expansion of the far groups' series.  Warp v takes the far groups
-// v, v + 4, ... of the box (lane n holds its partial L_n and L_{n+32}); the
-// four partials are added in warp order.
-__global__ void __launch_bounds__(128)
+// C(n + k, n) for k < PC_P, n < PL_P.
+struct PanelBinom {
+    double v[PC_P][PL_P];
+};
+constexpr PanelBinom make_panel_binom() {
+    PanelBinom b{};
+    for (int n = 0; n < PL_P; ++n) {
+        double c = 1.0;
+        for (int k = 0; k < PC_P; ++k) {
+            b.v[k][n] = c;
+            c = c * (double)(n + k + 1) / (double)(k + 1);
+        }
+    }
+    return b;
+}
+__device__ const PanelBinom panel_binom = make_panel_binom();
+
+// d = a b + d of an 8 x 4 by 4 x 8 FP64 tile: a = A[lane/4][lane%4], b =
+// B[lane%4][lane/4], (d0, d1) = D[lane/4][2 (lane%4) + 0, 1].
+__device__ __forceinline__ void mma_f64(double &d0, double &d1, double a, double b) {
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+                 : "+d"(d0), "+d"(d1)
+                 : "d"(a), "d"(b));
+}
+
+__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
+    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+
+// The occupied boxes' near-group masks (mwords words) and local expansions of
+// their far groups' series, a warp per box.  The sums over k are the binomial
+// matrix (the same for every box and group, held by each warp as A fragments)
+// times the groups' beta_k = A_k (R / D)^k: four far groups are the eight columns
+// of B (real and imaginary parts), on the FP64 tensor cores; then lane (row n =
+// lane/4 + 8 t, group lane%4) scales its sums by (-rb / D)^n into its L_n.  The
+// binomials formed per CTA (36 divisions one after the other) and the sums as
+// scalar FMAs took 95 us for 1,790 boxes x 32 groups; this takes 29 (four
+// warps per box: 39, each box's loads of the groups' data being a serial chain).
+constexpr int PL_WARPS = 4;
+
+__global__ void __launch_bounds__(32 * PL_WARPS)
 k_panel_locals(int64_t ngroups, const PanelGroup *__restrict__ groups, const PanelGrid *gd,
-               const int *__restrict__ flags, int mwords, double2 *__restrict__ locals,
+               const int *__restrict__ boxes, int mwords, double2 *__restrict__ locals,
                unsigned *__restrict__ masks) {
-    __shared__ double s_bin[PC_P][PL_P];  // [k - 1][n] = C(n + k - 1, n): lanes read rows
-    __shared__ double2 s_beta[4][PC_P];   // per warp: A_k (R / D)^k
+    constexpr int MT = PL_P / 8, KS = PC_P / 4;
+    static_assert(PL_P % 8 == 0 && PC_P % 4 == 0, "whole tiles");
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    for (int nn = threadIdx.x; nn < PL_P; nn += blockDim.x) {
-        double c = 1.0;  // C(n, n)
-        for (int k = 1; k <= PC_P; ++k) {
-            s_bin[k - 1][nn] = c;
-            c = c * (double)(nn + k) / (double)k;  // C(n + k, n)
-        }
-    }
-    __shared__ double2 s_part[4][PL_P];
-    const int box = blockIdx.x;
-    if (!flags[box]) return;  // the whole CTA: no point there
-    __syncthreads();
-    const int bx = box / PL_NB, by = box - bx * PL_NB;
-    const double wb = gd->wb;
-    const double zbx = gd->x0 + ((double)bx + 0.5) * wb, zby = gd->y0 + ((double)by + 0.5) * wb;
-    const double rb = 0.70710678118654757 * wb;
-    double2 l0 = make_double2(0.0, 0.0), l1 = make_double2(0.0, 0.0);  // L_lane, L_lane+32
-    for (int w = 0; w < mwords; ++w) {
-        const int64_t g = (int64_t)w * 32 + lane;
-        bool near = false;
-        if (g < ngroups) {
-            const double dx = zbx - groups[g].cx, dy = zby - groups[g].cy;
-            const double R = groups[g].R;
-            const double d = sqrt(dx * dx + dy * dy);
-            near = !(d >= fmax(2.0 * R + rb, R + 2.0 * rb) * 1.0000001);
-        }
-        const unsigned nm = __ballot_sync(0xffffffffu, near);
-        const unsigned valid = __ballot_sync(0xffffffffu, g < ngroups);
-        if (wid == 0 && lane == 0) masks[(int64_t)box * mwords + w] = nm;
-        unsigned far = valid & ~nm;
-        // this warp's share: the (wid)-th, (wid + 4)-th, ... far group of the word
-        for (int skip = wid; skip > 0 && far; --skip) far &= far - 1;
-        while (far) {
-            const int j = __ffs(far) - 1;
-            far &= far - 1;
-            const PanelGroup &G = groups[(int64_t)w * 32 + j];
-            const double dx = zbx - G.cx, dy = zby - G.cy;
-            const double inv = 1.0 / (dx * dx + dy * dy);
-            const double rr = dx * inv, ri = -dy * inv;  // 1 / D
-            // beta_k = A_k (R / D)^k, k = lane + 1 (and lane + 33)
-            for (int k = lane + 1; k <= PC_P; k += 32) {
-                double pr = 1.0, pi = 0.0, br = G.R * rr, bi = G.R * ri;
-                for (int e = k; e; e >>= 1) {  // (R / D)^k by squaring
-                    if (e & 1) {
-                        const double t = pr * br - pi * bi;
-                        pi = pr * bi + pi * br;
-                        pr = t;
-                    }
-                    const double t = br * br - bi * bi;
-                    bi = 2.0 * br * bi;
-                    br = t;
-                }
-                const double2 a = G.a[k - 1];
-                s_beta[wid][k - 1] = make_double2(a.x * pr - a.y * pi, a.x * pi + a.y * pr);
-            }
-            __syncwarp();
-            // L_n += (-rb / D)^n sum_k C(n + k - 1, n) beta_k, for n = lane and
-            // n = lane + 32 in one pass over k (even and odd k summed apart)
-            const bool two = lane + 32 < PL_P;
-            const int n1 = two ? lane + 32 : lane;
-            double a0r = 0.0, a0i = 0.0, a1r = 0.0, a1i = 0.0;  // n = lane: even, odd k
-            double c0r = 0.0, c0i = 0.0, c1r = 0.0, c1i = 0.0;  // n = lane + 32
-#pragma unroll 6
-            for (int k = 0; k < PC_P; k += 2) {
-                const double2 b0 = s_beta[wid][k], b1 = s_beta[wid][k + 1];
-                const double e0 = s_bin[k][lane], e1 = s_bin[k + 1][lane];
-                a0r = fma(e0, b0.x, a0r);
-                a0i = fma(e0, b0.y, a0i);
-                a1r = fma(e1, b1.x, a1r);
-                a1i = fma(e1, b1.y, a1i);
-                const double f0 = s_bin[k][n1], f1 = s_bin[k + 1][n1];
-                c0r = fma(f0, b0.x, c0r);
-                c0i = fma(f0, b0.y, c0i);
-                c1r = fma(f1, b1.x, c1r);
-                c1i = fma(f1, b1.y, c1i);
-            }
+    const int nr = lane >> 2, kq = lane & 3;
+    double af[MT][KS];
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int n = h ? n1 : lane;
-                const double sr = h ? c0r + c1r : a0r + a1r, si = h ? c0i + c1i : a0i + a1i;
-                double pr = 1.0, pi = 0.0, br = -rb * rr, bi = -rb * ri;  // (-rb / D)^n
-                for (int e = n; e; e >>= 1) {
-                    if (e & 1) {
-                        const double t = pr * br - pi * bi;
-                        pi = pr * bi + pi * br;
-                        pr = t;
-                    }
-                    const double t = br * br - bi * bi;
-                    bi = 2.0 * br * bi;
-                    br = t;
-                }
-                const double vr = sr * pr - si * pi, vi = sr * pi + si * pr;
-                if (h == 0) l0 = make_double2(l0.x + vr, l0.y + vi);
-                else if (two) l1 = make_double2(l1.x + vr, l1.y + vi);
-            }
-            __syncwarp();  // s_beta is read before the next group refills it
-            for (int skip = 3; skip > 0 && far; --skip) far &= far - 1;  // the next 3: other warps
-        }
-    }
-    s_part[wid][lane] = l0;
-    if (lane + 32 < PL_P) s_part[wid][lane + 32] = l1;
-    __syncthreads();
-    if (wid == 0) {
-        double2 *L = locals + (int64_t)box * PL_P;
-        for (int n = lane; n < PL_P; n += 32) {
-            double2 v = s_part[0][n];
+    for (int t = 0; t < MT; ++t)
 #pragma unroll
-            for (int q = 1; q < 4; ++q) v = make_double2(v.x + s_part[q][n].x, v.y + s_part[q][n].y);
-            L[n] = v;
+        for (int s = 0; s < KS; ++s) af[t][s] = panel_binom.v[4 * s + kq][8 * t + nr];
+    const double wb = gd->wb, rb = 0.70710678118654757 * wb;
+    const int nocc = gd->nocc;
+    for (int k = wid * gridDim.x + blockIdx.x; k < nocc; k += PL_WARPS * gridDim.x) {
+        const int box = boxes[k];
+        const int bx = box / PL_NB, by = box - bx * PL_NB;
+        const double zbx = gd->x0 + ((double)bx + 0.5) * wb, zby = gd->y0 + ((double)by + 0.5) * wb;
+        double2 acc[MT];
+#pragma unroll
+        for (int t = 0; t < MT; ++t) acc[t] = make_double2(0.0, 0.0);
+        for (int w = 0; w < mwords; ++w) {
+            const int64_t g = (int64_t)w * 32 + lane;
+            bool near = false;
+            double2 p = make_double2(0.0, 0.0), u = make_double2(0.0, 0.0);  // R / D, -rb / D
+            if (g < ngroups) {
+                const double dx = zbx - groups[g].cx, dy = zby - groups[g].cy;
+                const double R = groups[g].R, d2 = dx * dx + dy * dy;
+                near = !(sqrt(d2) >= fmax(2.0 * R + rb, R + 2.0 * rb) * 1.0000001);
+                const double inv = 1.0 / d2;
+                p = make_double2(R * dx * inv, -R * dy * inv);
+                u = make_double2(-rb * dx * inv, rb * dy * inv);
+            }
+            const unsigned nm = __ballot_sync(0xffffffffu, near);
+            const unsigned valid = __ballot_sync(0xffffffffu, g < ngroups);
+            if (lane == 0) masks[(int64_t)box * mwords + w] = nm;
+            unsigned far = valid & ~nm;
+            while (far) {
+                int src[4];  // the batch's groups within the word, -1 past the last
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    src[q] = __ffs(far) - 1;
+                    far &= far - 1;
+                }
+                const int bq = lane >> 3, part = nr & 1;  // B column: group and part
+                const int sb = bq == 0 ? src[0] : bq == 1 ? src[1] : bq == 2 ? src[2] : src[3];
+                const int sd = kq == 0 ? src[0] : kq == 1 ? src[1] : kq == 2 ? src[2] : src[3];
+                const double2 p1 = make_double2(__shfl_sync(0xffffffffu, p.x, max(sb, 0)),
+                                                __shfl_sync(0xffffffffu, p.y, max(sb, 0)));
+                const double2 u1 = make_double2(__shfl_sync(0xffffffffu, u.x, max(sd, 0)),
+                                                __shfl_sync(0xffffffffu, u.y, max(sd, 0)));
+                // beta_k for k = kq + 1, kq + 5, ..
+                const double2 p2 = cmul(p1, p1), p4 = cmul(p2, p2);
+                double2 pw = kq == 0 ? p1 : kq == 1 ? p2 : kq == 2 ? cmul(p2, p1) : p4;
+                const double2 *A = groups[(int64_t)w * 32 + max(sb, 0)].a;
+                double b[KS];
+#pragma unroll
+                for (int s = 0; s < KS; ++s) {
+                    const double2 a = A[4 * s + kq];
+                    const double v = part ? fma(a.x, pw.y, a.y * pw.x) : fma(a.x, pw.x, -(a.y * pw.y));
+                    b[s] = sb >= 0 ? v : 0.0;
+                    pw = cmul(pw, p4);
+                }
+                // (-rb / D)^n for n = nr, nr + 8, .. of group kq's column
+                const double2 u2 = cmul(u1, u1), u4 = cmul(u2, u2), u8 = cmul(u4, u4);
+                double2 un = nr & 1 ? u1 : make_double2(1.0, 0.0);
+                if (nr & 2) un = cmul(un, u2);
+                if (nr & 4) un = cmul(un, u4);
+                double d0[MT], d1[MT];
+#pragma unroll
+                for (int t = 0; t < MT; ++t) d0[t] = d1[t] = 0.0;
+#pragma unroll
+                for (int s = 0; s < KS; ++s)  // the rows' chains side by side
+#pragma unroll
+                    for (int t = 0; t < MT; ++t) mma_f64(d0[t], d1[t], af[t][s], b[s]);
+#pragma unroll
+                for (int t = 0; t < MT; ++t) {
+                    if (sd >= 0) {
+                        acc[t].x += d0[t] * un.x - d1[t] * un.y;
+                        acc[t].y += d0[t] * un.y + d1[t] * un.x;
+                    }
+                    un = cmul(un, u8);
+                }
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < MT; ++t) {
+#pragma unroll
+            for (int o = 1; o <= 2; o <<= 1) {
+                acc[t].x += __shfl_xor_sync(0xffffffffu, acc[t].x, o);
+                acc[t].y += __shfl_xor_sync(0xffffffffu, acc[t].y, o);
+            }
+            if (kq == 0) locals[(int64_t)box * PL_P + 8 * t + nr] = acc[t];
         }
     }
 }
@@ -547,15 +689,19 @@ k_panel_velocity_boxed(int64_t ngroups, const PanelGroup *__restrict__ groups,
                        double *__restrict__ vx, double *__restrict__ vy, int accumulate,
                        float log2_tol, const PanelGrid *gd, int mwords,
                        const double2 *__restrict__ locals, const unsigned *__restrict__ masks,
-                       const PanelGroup *__restrict__ subs) {
+                       const PanelGroup *__restrict__ subs, const double2 *__restrict__ pts,
+                       const int32_t *__restrict__ idx) {
     const double x0 = gd->x0, y0 = gd->y0, wb = gd->wb;
     const double rb = 0.70710678118654757 * wb, irb = 1.0 / rb;
-    for (int64_t i = (int64_t)blockIdx.x * PN_THREADS + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * PN_THREADS) {
-        const double px = xv[i], py = yv[i];
-        const int bx = min(max((int)floor((px - x0) / wb), 0), PL_NB - 1);
-        const int by = min(max((int)floor((py - y0) / wb), 0), PL_NB - 1);
-        const int box = bx * PL_NB + by;
+    const bool sorted = gd->sorted;
+    for (int64_t j = (int64_t)blockIdx.x * PN_THREADS + threadIdx.x; j < n;
+         j += (int64_t)gridDim.x * PN_THREADS) {
+        const int64_t i = sorted ? (int64_t)idx[j] : j;
+        if (!PF_IDX_OK(i, n, 302)) continue;
+        const double2 pt = sorted ? pts[j] : make_double2(xv[i], yv[i]);
+        const double px = pt.x, py = pt.y;
+        const int box = panel_box(px, py, x0, y0, wb);
+        const int bx = box / PL_NB, by = box - bx * PL_NB;
         // the far groups: sum_n L_n u^n, u = (z - zb) / rb
         const double ur = (px - (x0 + ((double)bx + 0.5) * wb)) * irb;
         const double ui = (py - (y0 + ((double)by + 0.5) * wb)) * irb;
@@ -692,6 +838,14 @@ static pf_status panel_velocity(pf_ctx *ctx, const char *name, int64_t m, const 
         }
         return PF_OK;
     }
+    // slices of the points: bounds the per-point scratch (28 bytes each)
+    if (n > PL_SLICE) {
+        for (int64_t i = 0; i < n; i += PL_SLICE)
+            PF_TRY(panel_velocity(ctx, name, m, gamma, xs, ys, xe, ye, cosa, sina,
+                                  std::min<int64_t>(PL_SLICE, n - i), xv + i, yv + i, vx + i, vy + i,
+                                  accumulate, stream, source));
+        return PF_OK;
+    }
     const int64_t ngroups = pf::ceil_div(m, PC_G);
     const size_t gbytes = sizeof(PanelGroup) * (size_t)ngroups;
     const size_t pbytes = sizeof(PanelSm) * (size_t)m;
@@ -701,37 +855,50 @@ static pf_status panel_velocity(pf_ctx *ctx, const char *name, int64_t m, const 
     const int mwords = (int)pf::ceil_div(ngroups, (int64_t)32);
     const size_t lbytes = boxed ? sizeof(double2) * PL_P * PL_NB * PL_NB : 0;
     const size_t mbytes = boxed ? sizeof(unsigned) * (size_t)mwords * PL_NB * PL_NB : 0;
-    const size_t fbytes = boxed ? sizeof(int) * PL_NB * PL_NB : 0;
+    // counts, starts, occupied boxes, and the counting CTAs' bases
+    const size_t fbytes = boxed ? (3 + (size_t)ctx->num_sms) * sizeof(int) * PL_NB * PL_NB : 0;
+    // per point: box and rank, then (points without order) coordinates and index
+    const size_t wbytes = boxed ? sizeof(int2) * (size_t)n : 0;
+    const size_t qbytes = boxed ? sizeof(double2) * (size_t)n : 0;
+    const size_t ibytes = boxed ? sizeof(int32_t) * (size_t)n : 0;
     const int64_t nsubs = pf::ceil_div(m, (int64_t)PL_SUB);
     const size_t sbytes = boxed ? sizeof(PanelGroup) * (size_t)nsubs : 0;
     PF_TRY(pf::arena_reserve(ctx, pf::align256(gbytes) + pf::align256(pbytes) +
                                       (boxed ? pf::align256(sizeof(PanelGrid)) +
                                                    pf::align256(lbytes) + pf::align256(mbytes) +
-                                                   pf::align256(fbytes) + pf::align256(sbytes)
+                                                   pf::align256(fbytes) + pf::align256(sbytes) +
+                                                   pf::align256(wbytes) + pf::align256(qbytes) +
+                                                   pf::align256(ibytes)
                                              : 0)));
     auto *groups = static_cast<PanelGroup *>(pf::arena_take(ctx, gbytes));
     auto *pan = static_cast<PanelSm *>(pf::arena_take(ctx, pbytes));
     PanelGrid *gd = nullptr;
     double2 *locals = nullptr;
     unsigned *masks = nullptr;
-    int *flags = nullptr;
+    int *counts = nullptr;
     PanelGroup *subs = nullptr;
+    int2 *where = nullptr;
+    double2 *pts = nullptr;
+    int32_t *idx = nullptr;
     if (boxed) {
         gd = static_cast<PanelGrid *>(pf::arena_take(ctx, sizeof(PanelGrid)));
         locals = static_cast<double2 *>(pf::arena_take(ctx, lbytes));
         masks = static_cast<unsigned *>(pf::arena_take(ctx, mbytes));
-        flags = static_cast<int *>(pf::arena_take(ctx, fbytes));
+        counts = static_cast<int *>(pf::arena_take(ctx, fbytes));
         subs = static_cast<PanelGroup *>(pf::arena_take(ctx, sbytes));
+        where = static_cast<int2 *>(pf::arena_take(ctx, wbytes));
+        pts = static_cast<double2 *>(pf::arena_take(ctx, qbytes));
+        idx = static_cast<int32_t *>(pf::arena_take(ctx, ibytes));
     }
-    if (!groups || !pan || (boxed && (!gd || !locals || !masks || !flags || !subs))) {
+    if (!groups || !pan || (boxed && (!gd || !locals || !masks || !counts || !subs || !where || !pts || !idx))) {
         pf::set_error("%s: scratch too small", name);
         return PF_ERR_OOM;
     }
     if (source)
-        k_panel_groups<true><<<(unsigned)ngroups, 32, 0, st>>>(m, gamma, xs, ys, xe, ye, cosa,
+        k_panel_groups<true><<<(unsigned)ngroups, 64, 0, st>>>(m, gamma, xs, ys, xe, ye, cosa,
                                                                sina, groups, pan);
     else
-        k_panel_groups<false><<<(unsigned)ngroups, 32, 0, st>>>(m, gamma, xs, ys, xe, ye, cosa,
+        k_panel_groups<false><<<(unsigned)ngroups, 64, 0, st>>>(m, gamma, xs, ys, xe, ye, cosa,
                                                                 sina, groups, pan);
     PF_TRY(pf::launch_status("k_panel_groups"));
     // persistent grid: a few CTAs per SM, each over many blocks of points
@@ -740,10 +907,10 @@ static pf_status panel_velocity(pf_ctx *ctx, const char *name, int64_t m, const 
     const float log2_tol = (float)std::log2(PC_EPS * (1.0 - PC_RHO) / 2.0);
     if (boxed) {
         if (source)
-            k_panel_groups<true, PL_SUB><<<(unsigned)nsubs, 32, 0, st>>>(
+            k_panel_groups<true, PL_SUB><<<(unsigned)nsubs, 64, 0, st>>>(
                 m, gamma, xs, ys, xe, ye, cosa, sina, subs, nullptr);
         else
-            k_panel_groups<false, PL_SUB><<<(unsigned)nsubs, 32, 0, st>>>(
+            k_panel_groups<false, PL_SUB><<<(unsigned)nsubs, 64, 0, st>>>(
                 m, gamma, xs, ys, xe, ye, cosa, sina, subs, nullptr);
         PF_TRY(pf::launch_status("k_panel_groups"));
         k_panel_grid_init<<<1, 1, 0, st>>>(gd);
@@ -752,20 +919,28 @@ static pf_status panel_velocity(pf_ctx *ctx, const char *name, int64_t m, const 
         PF_TRY(pf::launch_status("k_panel_bbox"));
         k_panel_grid_set<<<1, 1, 0, st>>>(gd);
         PF_TRY(pf::launch_status("k_panel_grid_set"));
-        PF_CUDA_TRY(cudaMemsetAsync(flags, 0, fbytes, st));
-        k_panel_flags<<<(unsigned)grid, PN_THREADS, 0, st>>>(n, xv, yv, gd, flags);
-        PF_TRY(pf::launch_status("k_panel_flags"));
-        k_panel_locals<<<PL_NB * PL_NB, 128, 0, st>>>(ngroups, groups, gd, flags, mwords, locals,
-                                                      masks);
+        int *const start = counts + PL_NB * PL_NB, *const boxes = start + PL_NB * PL_NB;
+        int *const base = boxes + PL_NB * PL_NB;
+        PF_CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int) * PL_NB * PL_NB, st));
+        k_panel_count<<<(unsigned)ctx->num_sms, PCT_THREADS, 0, st>>>(n, xv, yv, gd, counts, where,
+                                                                      base);
+        PF_TRY(pf::launch_status("k_panel_count"));
+        k_panel_starts<<<1, 1024, 0, st>>>(n, gd, counts, start, boxes);
+        PF_TRY(pf::launch_status("k_panel_starts"));
+        k_panel_place<<<(unsigned)ctx->num_sms, PCT_THREADS, 0, st>>>(n, gd, xv, yv, where, base,
+                                                                      start, pts, idx);
+        PF_TRY(pf::launch_status("k_panel_place"));
+        k_panel_locals<<<(unsigned)(ctx->num_sms * 2), 32 * PL_WARPS, 0, st>>>(
+            ngroups, groups, gd, boxes, mwords, locals, masks);
         PF_TRY(pf::launch_status("k_panel_locals"));
         if (source)
             k_panel_velocity_boxed<true><<<(unsigned)grid, PN_THREADS, 0, st>>>(
                 ngroups, groups, pan, m, n, xv, yv, vx, vy, accumulate, log2_tol, gd, mwords,
-                locals, masks, subs);
+                locals, masks, subs, pts, idx);
         else
             k_panel_velocity_boxed<false><<<(unsigned)grid, PN_THREADS, 0, st>>>(
                 ngroups, groups, pan, m, n, xv, yv, vx, vy, accumulate, log2_tol, gd, mwords,
-                locals, masks, subs);
+                locals, masks, subs, pts, idx);
         return pf::launch_status("k_panel_velocity_boxed");
     }
     if (source)

@@ -195,3 +195,33 @@ def test_box_grid_path_as_accurate_as_per_point_path(m, shuffle):
     rx, ry = oracle.panel_velocity(*arrs, xv, yv)
     e_box, e_pt = normwise_err(vx, vy, rx, ry), normwise_err(px, py, rx, ry)
     assert e_box <= TOL and e_box <= 1.5 * e_pt + 1e-10, (e_box, e_pt)
+
+
+@pytest.mark.parametrize("n,m", [(32768, 128), (32769, 130), (50001, 200), (200003, 512)])
+def test_box_order_gives_the_input_orders_values(n, m):
+    """Points in an order that stays in a box for long are evaluated in place,
+    unordered ones in box order: the same points sorted into grid cells and
+    shuffled give bitwise the same velocities (a point's arithmetic does not
+    depend on the order), and
+    so does accumulation onto given velocities."""
+    import pfblob
+    from pfblob import workloads as wl
+    ps = wl.cylinder_panels(m)
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()
+    arrs = [dev(a) for a in (ps.gamma, ps.xs, ps.ys, ps.xe, ps.ye, ps.cosa, ps.sina)]
+    xv, yv = _annulus(n, 1.0, 1.5, n)
+    cell = np.floor((xv + 1.5) / 3.0 * 64) * 64 + np.floor((yv + 1.5) / 3.0 * 64)
+    order = np.argsort(cell, kind="stable")
+    xs, ys = dev(xv[order]), dev(yv[order])
+    ax, ay = pfblob.inducedVelocity(*arrs, xs, ys)
+    shuf = torch.randperm(n, device="cuda", generator=torch.Generator("cuda").manual_seed(n))
+    bx, by = pfblob.inducedVelocity(*arrs, xs[shuf].contiguous(), ys[shuf].contiguous())
+    assert torch.equal(ax[shuf], bx) and torch.equal(ay[shuf], by)
+    cx, cy = torch.ones_like(bx), torch.full_like(by, -2.0)
+    pfblob.panel_velocity_device(*arrs, xs[shuf].contiguous(), ys[shuf].contiguous(), cx, cy,
+                                 accumulate=True)
+    assert torch.equal(cx, bx + 1.0) and torch.equal(cy, by - 2.0)
+    rx, ry = oracle.panel_velocity(ps.gamma, ps.xs, ps.ys, ps.xe, ps.ye, ps.cosa, ps.sina,
+                                   xv[:2000].copy(), yv[:2000].copy())
+    inv = np.argsort(order)[:2000]
+    assert normwise_err(ax.cpu().numpy()[inv], ay.cpu().numpy()[inv], rx, ry) <= TOL
