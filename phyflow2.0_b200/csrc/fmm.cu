@@ -1543,7 +1543,7 @@ pf_status velocity_fmm(pf_ctx *ctx, int64_t n_src, const double *x, const double
         BBox *bb = static_cast<BBox *>(pf::arena_take(ctx, sizeof(BBox)));
         k_bbox_init<<<1, 1, 0, st>>>(bb);
         PF_TRY(pf::launch_status("k_bbox_init"));
-        const int cap = ctx->num_sms * 8;
+        const int cap = ctx->num_sms * 4;  // each CTA ends in five atomics on the same words
         k_bbox<<<(unsigned)std::min<int64_t>(pf::ceil_div(n_src, 256), cap), 256, 0, st>>>(
             x, y, n_src, bb);
         PF_TRY(pf::launch_status("k_bbox"));

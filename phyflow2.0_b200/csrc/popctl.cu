@@ -80,10 +80,22 @@ k_pc_loss(int64_t n, const int64_t *__restrict__ n_dev, const double *__restrict
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    if (threadIdx.x < PC_DECADES) {
+    {  // thread (q, k): decade k of the CTAs q, q + 16, ... in order; then over q
+       // (one thread per decade over all 592 CTAs took most of the launch's 23 us)
+        constexpr int PARTS = PC_THREADS / PC_DECADES;
+        __shared__ double s_part[PARTS][PC_DECADES];
+        const int k = threadIdx.x % PC_DECADES, q = threadIdx.x / PC_DECADES;
         double s = 0.0;
-        for (int b = 0; b < (int)gridDim.x; ++b) s += __ldcg(&part[b * PC_DECADES + threadIdx.x]);
-        s_tot[threadIdx.x] = s;
+#pragma unroll 8
+        for (int b = q; b < (int)gridDim.x; b += PARTS) s += __ldcg(&part[b * PC_DECADES + k]);
+        s_part[q][k] = s;
+        __syncthreads();
+        if (threadIdx.x < PC_DECADES) {
+            s = 0.0;
+#pragma unroll
+            for (int v = 0; v < PARTS; ++v) s += s_part[v][threadIdx.x];
+            s_tot[threadIdx.x] = s;
+        }
     }
     __syncthreads();
     if (threadIdx.x == 0) {

@@ -21,8 +21,8 @@
 //   4. k_rm_place  : blob -> its slot in cell order: a 32-byte record {x/h,
 //      y/h, g, index} (the IEEE quotients of _regridding.py:183 computed once
 //      per blob; x, y for Tutty).
-//   5. seg_sort_listed + k_rm_stencil_big : cells of more than SEG_SMALL blobs
-//      (dense clusters), one CTA per cell, stencil partial sums to a side table.
+//   5. k_rm_big : cells of more than SEG_SMALL blobs (dense clusters), one CTA per
+//      cell, stencil partial sums to a side table.
 //   6. k_rm_tile   : one CTA per tile of 8 x 29 output cells.  Each thread
 //      takes one of the 11 x 32 base cells feeding the tile (a warp per base
 //      row), walks the cell's blobs in input-index order (found in
@@ -34,8 +34,8 @@
 //      cells that cover it in fixed (b, a) order and writes x = ix*h + 0.5h +
 //      xb0 (same order as :217-218), g, ix, iy at its slot.
 //      [pf_remesh_population_control: the cell values and flags go to HBM
-//       instead, PopulationControl (popctl.cu) clears the flags of the dropped
-//       cells, then a scan and k_rm_emit.]
+//       instead, PopulationControl (popctl.cu) finds the threshold, then
+//       k_rm_keep_count and k_rm_keep_emit write the kept cells.]
 //   7. k_rm_finish : output count and status words.
 // No floating-point atomics: each partial and each output value is produced
 // by one thread in a fixed order, so results are bitwise reproducible.
@@ -47,7 +47,6 @@
 #include <vector>
 
 #include "remesh.cuh"
-#include "scan.cuh"
 #include "segsort.cuh"
 
 namespace {
@@ -56,6 +55,10 @@ using pf::RM_IDX_OFF;
 using pf::RmHead;
 
 constexpr int RM_THREADS = 256;
+// CTAs per SM of the grid-stride passes that end in atomics on shared words (the
+// extent, the moments' ticket): 2^20 blobs, k_rm_extent 11.6 / 9.3 / 10.8 us and
+// k_rm_place 19.1 / 16.4 / 19.3 us with 8 / 4 / 2
+constexpr int RM_CTAS = 4;
 constexpr int32_t IDX_LIMIT = 1 << 30;
 
 // scan tiles
@@ -620,21 +623,6 @@ k_rm_place(int64_t n, RmHead *hd, const int32_t *__restrict__ cell,
     grid_moments<RM_THREADS>(m, mpart, &hd->ticket_in, hd->mom);
 }
 
-// The input indices of each listed cell of more than SEG_SMALL blobs, from its
-// records into vals[start ..] (for the segment sort).
-__global__ void __launch_bounds__(RM_THREADS)
-k_rm_big_gather(const int32_t *__restrict__ list, const RmHead *__restrict__ hd,
-                const int32_t *__restrict__ start, const int32_t *__restrict__ count,
-                const WRec *__restrict__ recs, int32_t *__restrict__ vals) {
-    if (!hd->ok) return;
-    const int nlist = hd->big_n;
-    for (int k = blockIdx.x; k < nlist; k += gridDim.x) {
-        const int64_t bc = list[k];
-        const int cnt = count[bc], s0 = start[bc];
-        for (int j = threadIdx.x; j < cnt; j += RM_THREADS) vals[s0 + j] = (int32_t)recs[s0 + j].idx;
-    }
-}
-
 // Weights of the tile kernel: M4' with any c, M4' with c = 0, Tutty.
 constexpr int WK_M4 = 0, WK_M4_PLAIN = 1, WK_TUTTY = 2;
 
@@ -682,41 +670,52 @@ __device__ __forceinline__ void rec_w8(double v1, double v2, int64_t ix0, int64_
     }
 }
 
-// The stencil of each listed cell of more than SEG_SMALL blobs (sorted by
-// seg_sort_listed), one CTA per cell: thread t sums the blobs t, t + RM_THREADS,
-// ... of the cell (in cell order), then the CTA adds the threads' partial sums
-// in a fixed tree order into part_big[16 k ..].  The cell's count is then
-// replaced by -(k + 1), which is how k_rm_tile finds the table entry.
+// The stencil of each listed cell of more than SEG_SMALL blobs, one CTA per cell:
+// the cell's input indices from its records are put in order, then thread t <
+// RM_THREADS sums the blobs t, t + RM_THREADS, ... of the cell, and the CTA adds
+// the threads' partial sums in a fixed tree order into part_big[16 k ..].  The
+// cell's count is then replaced by -(k + 1), which is how k_rm_tile finds the
+// table entry.  (One launch: without such cells -- the usual set -- it ends at
+// once, and gathering, sorting and summing as three cost a launch each.)
 template <bool TUTTY>
-__global__ void __launch_bounds__(RM_THREADS)
-k_rm_stencil_big(const int32_t *__restrict__ list, const RmHead *__restrict__ hd,
-                 const int32_t *__restrict__ start, int32_t *__restrict__ count,
-                 const int32_t *__restrict__ perm, const double *__restrict__ x,
-                 const double *__restrict__ y, const double *__restrict__ g, WParams wp,
-                 double *__restrict__ part_big) {
-    __shared__ double s_p[16][RM_THREADS];
+__global__ void __launch_bounds__(SEG_THREADS)
+k_rm_big(const int32_t *__restrict__ list, const RmHead *__restrict__ hd,
+         const int32_t *__restrict__ start, int32_t *__restrict__ count,
+         const WRec *__restrict__ recs, int32_t *__restrict__ vals, int32_t *__restrict__ tmp,
+         const double *__restrict__ x, const double *__restrict__ y, const double *__restrict__ g,
+         WParams wp, double *__restrict__ part_big) {
+    // the sort's values, then the threads' sums
+    __shared__ __align__(16) unsigned char s_mem[16 * RM_THREADS * sizeof(double)];
+    static_assert(SEG_CHUNK * sizeof(int32_t) <= sizeof(s_mem), "the sort's chunk fits");
     Win w;
     if (!load_win(hd, w)) return;
+    int32_t *const s_v = reinterpret_cast<int32_t *>(s_mem);
+    double(*const s_p)[RM_THREADS] = reinterpret_cast<double(*)[RM_THREADS]>(s_mem);
     const int nlist = hd->big_n;
     for (int k = blockIdx.x; k < nlist; k += gridDim.x) {
         const int64_t bc = list[k];
         const int cnt = count[bc], s0 = start[bc];
+        for (int j = threadIdx.x; j < cnt; j += SEG_THREADS) vals[s0 + j] = (int32_t)recs[s0 + j].idx;
+        __syncthreads();
+        seg_sort_block(vals + s0, tmp + s0, cnt, s_v);
         const int64_t bx = bc / w.nby, by = bc - bx * w.nby;
-        double p[16];
+        if (threadIdx.x < RM_THREADS) {
+            double p[16];
 #pragma unroll
-        for (int q = 0; q < 16; ++q) p[q] = 0.0;
-        for (int j = threadIdx.x; j < cnt; j += RM_THREADS) {
-            const int32_t i = perm[s0 + j];
-            const double gv = g[i];
-            double wx[4], wy[4];
-            blob_w8<TUTTY>(x[i], y[i], lat_x(w, bx), lat_y(w, by), wp, wx, wy);
+            for (int q = 0; q < 16; ++q) p[q] = 0.0;
+            for (int j = threadIdx.x; j < cnt; j += RM_THREADS) {
+                const int32_t i = vals[s0 + j];
+                const double gv = g[i];
+                double wx[4], wy[4];
+                blob_w8<TUTTY>(x[i], y[i], lat_x(w, bx), lat_y(w, by), wp, wx, wy);
 #pragma unroll
-            for (int a = 0; a < 4; ++a)
+                for (int a = 0; a < 4; ++a)
 #pragma unroll
-                for (int b = 0; b < 4; ++b) p[a * 4 + b] += (wx[a] * wy[b]) * gv;
+                    for (int b = 0; b < 4; ++b) p[a * 4 + b] += (wx[a] * wy[b]) * gv;
+            }
+#pragma unroll
+            for (int q = 0; q < 16; ++q) s_p[q][threadIdx.x] = p[q];
         }
-#pragma unroll
-        for (int q = 0; q < 16; ++q) s_p[q][threadIdx.x] = p[q];
         __syncthreads();
         for (int s = RM_THREADS / 2; s > 0; s >>= 1) {
             if ((int)threadIdx.x < s)
@@ -1036,29 +1035,111 @@ cudaError_t tile_smem_attr() {
     return e;
 }
 
-// cells mode: emit the flagged cells at their slots (cid up to the capacity;
-// flags beyond the window are zero)
-__global__ void __launch_bounds__(RM_THREADS)
-k_rm_emit(int64_t cap_cell, const RmHead *__restrict__ hd, WParams wp,
-          const int32_t *__restrict__ flag, const int32_t *__restrict__ slot,
-          const double *__restrict__ acc, int64_t capacity, double *__restrict__ xo,
-          double *__restrict__ yo, double *__restrict__ go, int64_t *__restrict__ ixo,
-          int64_t *__restrict__ iyo) {
+// Cells mode: the touched cells that population control keeps (|value| not below
+// the threshold found), in cell order.  Two launches: k_rm_keep_count counts the
+// kept cells of each part of KP_TILE cells; k_rm_keep_emit adds the earlier
+// parts' counts itself, ranks its cells by ballots and writes the new blobs.
+// (Flags, a three-pass scan of slots and the emission as five launches took 25
+// us for 711,000 cells; these take 14.)
+constexpr int KP_THREADS = 256;
+constexpr int KP_STEPS = 8;  // 32 cells per warp and step
+constexpr int KP_TILE = KP_THREADS * KP_STEPS;
+
+__device__ __forceinline__ unsigned keep_ballot(const Win &w, int64_t cid,
+                                                const int32_t *__restrict__ flag,
+                                                const double *__restrict__ acc, double thr,
+                                                double &v) {
+    bool keep = false;
+    v = 0.0;
+    if (cid < w.ncell) {
+        v = acc[cid];
+        keep = flag[cid] != 0 && !(fabs(v) < thr);
+    }
+    return __ballot_sync(0xffffffffu, keep);
+}
+
+__global__ void __launch_bounds__(KP_THREADS)
+k_rm_keep_count(const RmHead *__restrict__ hd, const int32_t *__restrict__ flag,
+                const double *__restrict__ acc, const pf::PcState *__restrict__ pc,
+                int32_t *__restrict__ tsum) {
+    __shared__ int s_w[KP_THREADS / 32];
     Win w;
     if (!load_win(hd, w)) return;
-    const int64_t cid = (int64_t)blockIdx.x * RM_THREADS + threadIdx.x;
-    if (cid >= cap_cell || cid >= w.ncell) return;
-    if ((int64_t)hd->total > capacity) return;  // capacity error: write nothing
-    if (!flag[cid]) return;
-    const int64_t ox = cid / w.noy, oy = cid - ox * w.noy;
-    const int64_t ix = lat_x(w, ox), iy = lat_y(w, oy);
-    const int64_t p = slot[cid];
-    if (!PF_IDX_OK(p, capacity, 107)) return;
-    xo[p] = __dadd_rn(__dadd_rn(__dmul_rn((double)ix, wp.h), wp.h05), wp.xb0);
-    yo[p] = __dadd_rn(__dadd_rn(__dmul_rn((double)iy, wp.h), wp.h05), wp.yb0);
-    go[p] = acc[cid];
-    if (ixo) ixo[p] = ix;
-    if (iyo) iyo[p] = iy;
+    const int64_t t0 = (int64_t)blockIdx.x * KP_TILE;
+    if (t0 >= w.ncell) return;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const double thr = pc->thr;
+    int n = 0;
+    double v;
+#pragma unroll
+    for (int k = 0; k < KP_STEPS; ++k)
+        n += __popc(keep_ballot(w, t0 + (wid * KP_STEPS + k) * 32 + lane, flag, acc, thr, v));
+    if (lane == 0) s_w[wid] = n;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int k = 1; k < KP_THREADS / 32; ++k) n += s_w[k];
+        tsum[blockIdx.x] = n;
+    }
+}
+
+__global__ void __launch_bounds__(KP_THREADS)
+k_rm_keep_emit(RmHead *__restrict__ hd, WParams wp, const int32_t *__restrict__ flag,
+               const double *__restrict__ acc, const pf::PcState *__restrict__ pc,
+               const int32_t *__restrict__ tsum, int64_t capacity, double *__restrict__ xo,
+               double *__restrict__ yo, double *__restrict__ go, int64_t *__restrict__ ixo,
+               int64_t *__restrict__ iyo) {
+    __shared__ int s_w[KP_THREADS / 32], s_pre[KP_THREADS / 32], s_tot[KP_THREADS / 32];
+    Win w;
+    if (!load_win(hd, w)) return;
+    const int64_t t0 = (int64_t)blockIdx.x * KP_TILE;
+    if (t0 >= w.ncell) return;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const double thr = pc->thr;
+    const int ntiles = (int)((w.ncell + KP_TILE - 1) / KP_TILE);
+    int pre = 0, tot = 0;  // kept cells of the earlier parts, and of all
+    for (int j = threadIdx.x; j < ntiles; j += KP_THREADS) {
+        const int c = tsum[j];
+        tot += c;
+        if (j < (int)blockIdx.x) pre += c;
+    }
+    double v[KP_STEPS];
+    unsigned m[KP_STEPS];
+    int n = 0;
+#pragma unroll
+    for (int k = 0; k < KP_STEPS; ++k) {
+        m[k] = keep_ballot(w, t0 + (wid * KP_STEPS + k) * 32 + lane, flag, acc, thr, v[k]);
+        n += __popc(m[k]);
+    }
+    pre = __reduce_add_sync(0xffffffffu, pre);
+    tot = __reduce_add_sync(0xffffffffu, tot);
+    if (lane == 0) {
+        s_w[wid] = n;
+        s_pre[wid] = pre;
+        s_tot[wid] = tot;
+    }
+    __syncthreads();
+    int64_t at = 0, all = 0;
+#pragma unroll
+    for (int k = 0; k < KP_THREADS / 32; ++k) {
+        at += s_pre[k] + (k < wid ? s_w[k] : 0);
+        all += s_tot[k];
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) hd->total = (int32_t)all;
+    if (all > capacity) return;  // capacity error: write nothing
+#pragma unroll
+    for (int k = 0; k < KP_STEPS; ++k) {
+        const int64_t p = at + __popc(m[k] & ((1u << lane) - 1u));
+        at += __popc(m[k]);
+        if (!(m[k] >> lane & 1u) || !PF_IDX_OK(p, capacity, 107)) continue;
+        const int64_t cid = t0 + (wid * KP_STEPS + k) * 32 + lane;
+        const int64_t ox = cid / w.noy, oy = cid - ox * w.noy;
+        const int64_t ix = lat_x(w, ox), iy = lat_y(w, oy);
+        xo[p] = __dadd_rn(__dadd_rn(__dmul_rn((double)ix, wp.h), wp.h05), wp.xb0);
+        yo[p] = __dadd_rn(__dadd_rn(__dmul_rn((double)iy, wp.h), wp.h05), wp.yb0);
+        go[p] = v[k];
+        if (ixo) ixo[p] = ix;
+        if (iyo) iyo[p] = iy;
+    }
 }
 
 __global__ void k_rm_finish(const RmHead *__restrict__ hd, int32_t *__restrict__ total,
@@ -1104,8 +1185,7 @@ size_t remesh_scratch_bytes(int64_t n, int64_t cap_base, int64_t cap_cell, bool 
                align256(128 * big_slots(n)) + align256(32 * (ceil_div(n, RM_THREADS) + 1 + 2 * 1024 + 1)) +
                1024;
     if (cells_mode)
-        b += align256(4 * cap_cell) + align256(8 * cap_cell) +
-             align256(4 * scan_tmp_ints(cap_cell)) + popctl_scratch_bytes();
+        b += align256(4 * cap_cell) + align256(8 * cap_cell) + popctl_scratch_bytes();
     return b;
 }
 
@@ -1121,11 +1201,11 @@ pf_status remesh_core(Bump &sc, int64_t n, const double *x, const double *y, con
                   (long long)cap_base, (long long)cap_cell);
         return PF_ERR_INVALID_ARG;
     }
-    // head, counts (and flags in cells mode) first: one memset zeroes them
+    // head and counts first: one memset zeroes them
     RmHead *hd = (RmHead *)sc.take(sizeof(RmHead));
     int32_t *count = (int32_t *)sc.take(4 * cap_base);
     int32_t *flag = cells ? (int32_t *)sc.take(4 * cap_cell) : nullptr;
-    char *zero_end = cells ? (char *)(flag + cap_cell) : (char *)(count + cap_base);
+    char *zero_end = (char *)(count + cap_base);
     int32_t *cell = (int32_t *)sc.take(4 * n);
     int32_t *rank = (int32_t *)sc.take(4 * n);
     WRec *recs = (WRec *)sc.take(sizeof(WRec) * n);
@@ -1142,8 +1222,7 @@ pf_status remesh_core(Bump &sc, int64_t n, const double *x, const double *y, con
     const int64_t gn_max = ceil_div(n, RM_THREADS) + 1, gt_max = 2 * (int64_t)num_sms + 1;
     double *mpart = (double *)sc.take(32 * (gn_max + gt_max));
     double *acc = cells ? (double *)sc.take(8 * cap_cell) : nullptr;
-    int32_t *tmp = cells ? (int32_t *)sc.take(4 * scan_tmp_ints(cap_cell)) : nullptr;
-    if (!mpart || (cells && !tmp)) {
+    if (!mpart || (cells && !acc)) {
         set_error("remesh: scratch too small");
         return PF_ERR_OOM;
     }
@@ -1152,7 +1231,7 @@ pf_status remesh_core(Bump &sc, int64_t n, const double *x, const double *y, con
     PF_CUDA_TRY(cudaMemsetAsync(hd, 0, (size_t)(zero_end - (char *)hd), st));
     if (win.from_blobs) {
         int64_t grid = ceil_div(n, RM_THREADS);
-        const int64_t cap = (int64_t)num_sms * 8;
+        const int64_t cap = (int64_t)num_sms * RM_CTAS;
         if (grid > cap) grid = cap;
         if (grid < 1) grid = 1;
         k_rm_extent<<<(unsigned)grid, RM_THREADS, 0, st>>>(x, y, n, xb0, yb0, h2, h05, h, hd,
@@ -1183,7 +1262,7 @@ pf_status remesh_core(Bump &sc, int64_t n, const double *x, const double *y, con
         k_rm_scan_down<<<gsc, SC_THREADS, 0, st>>>(hd, count, ntA, tsA, tsB, oflag, start,
                                                   slot);
         PF_TRY(launch_status("k_rm_scan_down"));
-        const unsigned gp = (unsigned)std::min<int64_t>(gn, (int64_t)num_sms * 8);
+        const unsigned gp = (unsigned)std::min<int64_t>(gn, (int64_t)num_sms * RM_CTAS);
         if (tutty)
             k_rm_place<true><<<gp, RM_THREADS, 0, st>>>(n, hd, cell, rank, start, x, y, g, wp,
                                                         recs, bigc, mpart);
@@ -1191,19 +1270,15 @@ pf_status remesh_core(Bump &sc, int64_t n, const double *x, const double *y, con
             k_rm_place<false><<<gp, RM_THREADS, 0, st>>>(n, hd, cell, rank, start, x, y, g, wp,
                                                          recs, bigc, mpart);
         PF_TRY(launch_status("k_rm_place"));
-        // cells above SEG_SMALL blobs (dense clusters); the ranks are free now
+        // cells above SEG_SMALL blobs (dense clusters); the cell ids and ranks are free now
         const unsigned gbig = (unsigned)std::min<int64_t>(nbig, 64);
-        k_rm_big_gather<<<gbig, RM_THREADS, 0, st>>>(bigc, hd, start, count, recs, cell);
-        PF_TRY(launch_status("k_rm_big_gather"));
-        int32_t *perm = cell;  // the cell ids are no longer needed: sorted indices of big cells
-        PF_TRY(seg_sort_listed(bigc, &hd->big_n, start, count, perm, rank, nbig, st));
         if (tutty)
-            k_rm_stencil_big<true><<<gbig, RM_THREADS, 0, st>>>(bigc, hd, start, count, perm, x, y,
-                                                                g, wp, part_big);
+            k_rm_big<true><<<gbig, SEG_THREADS, 0, st>>>(bigc, hd, start, count, recs, cell, rank, x, y,
+                                                         g, wp, part_big);
         else
-            k_rm_stencil_big<false><<<gbig, RM_THREADS, 0, st>>>(bigc, hd, start, count, perm, x,
-                                                                 y, g, wp, part_big);
-        PF_TRY(launch_status("k_rm_stencil_big"));
+            k_rm_big<false><<<gbig, SEG_THREADS, 0, st>>>(bigc, hd, start, count, recs, cell, rank, x,
+                                                          y, g, wp, part_big);
+        PF_TRY(launch_status("k_rm_big"));
     }
     {
         // persistent: two CTAs per SM, at most one per tile of the capacity
@@ -1233,11 +1308,13 @@ pf_status remesh_core(Bump &sc, int64_t n, const double *x, const double *y, con
     }
     if (cells) {
         PF_TRY(popctl_decide(sc, cap_cell, acc, flag, *pc, st, &hd->ncell));
-        PF_TRY(popctl_flags(cap_cell, acc, flag, pc->state, flag, st));
-        PF_TRY(exclusive_scan_i32(flag, slot, cap_cell, tmp, &hd->total, st));
-        k_rm_emit<<<(unsigned)ceil_div(cap_cell, RM_THREADS), RM_THREADS, 0, st>>>(
-            cap_cell, hd, wp, flag, slot, acc, capacity, xo, yo, go, ixo, iyo);
-        PF_TRY(launch_status("k_rm_emit"));
+        // the slots' array is free in this mode: the parts' counts
+        const unsigned gk = (unsigned)ceil_div(cap_cell, KP_TILE);
+        k_rm_keep_count<<<gk, KP_THREADS, 0, st>>>(hd, flag, acc, pc->state, slot);
+        PF_TRY(launch_status("k_rm_keep_count"));
+        k_rm_keep_emit<<<gk, KP_THREADS, 0, st>>>(hd, wp, flag, acc, pc->state, slot, capacity, xo, yo,
+                                                  go, ixo, iyo);
+        PF_TRY(launch_status("k_rm_keep_emit"));
     }
     if (!total && !bad) return PF_OK;
     k_rm_finish<<<1, 1, 0, st>>>(hd, total, bad, nullptr, nullptr, nullptr, nullptr);
@@ -1368,14 +1445,15 @@ pf_status remesh_sync(pf_ctx *ctx, int64_t n, const double *x, const double *y, 
         PF_TRY(pf::remesh_core(sc, n, x, y, g, h, xb0, yb0, c, win, capacity, x_out, y_out, g_out,
                                ix_out, iy_out, nullptr, nullptr, st, ctx->num_sms,
                                popctl ? &pc : nullptr, kernel, &hd));
-        PF_CUDA_TRY(cudaMemcpyAsync(ctx->host_small, hd, sizeof(pf::RmHead),
+        // the decision and the head, one after the other in the scratch, in one copy
+        const size_t off = (size_t)((char *)hd - (char *)state);
+        PF_CUDA_TRY(cudaMemcpyAsync(ctx->host_small, state, off + sizeof(pf::RmHead),
                                     cudaMemcpyDeviceToHost, st));
-        if (popctl)
-            PF_CUDA_TRY(cudaMemcpyAsync(ctx->host_small + 8, &state->thr, sizeof(double),
-                                        cudaMemcpyDeviceToHost, st));
         PF_CUDA_TRY(cudaStreamSynchronize(st));
+        pf::PcState ps;
         pf::RmHead he;
-        memcpy(&he, ctx->host_small, sizeof(he));
+        memcpy(&ps, ctx->host_small, sizeof(ps));
+        memcpy(&he, (const char *)ctx->host_small + off, sizeof(he));
         if (he.bad & 1) {
             pf::set_error("pf_remesh: NaN or Inf blob coordinate");
             return PF_ERR_NAN_INPUT;
@@ -1409,7 +1487,7 @@ pf_status remesh_sync(pf_ctx *ctx, int64_t n, const double *x, const double *y, 
                                              std::min<int64_t>(nbx * nby + nbx * nby / 4, limit));
         const int64_t nout = he.ok ? he.total : 0;
         *n_out = nout;
-        if (popctl && thr_used) memcpy(thr_used, ctx->host_small + 8, sizeof(double));
+        if (popctl && thr_used) *thr_used = ps.thr;
         if (nout > capacity) {
             pf::set_error("pf_remesh: output needs %lld entries, capacity is %lld",
                           (long long)nout, (long long)capacity);

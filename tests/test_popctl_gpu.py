@@ -104,3 +104,23 @@ def test_blobs_evolve_fused_step_matches_separate_steps():
     xo, yo, go = pfblob.PopulationControl(xn, yn, gn, 1e-8, 1e-8)
     assert b.numBlobs == go.size
     assert np.array_equal(b.x, xo) and np.array_equal(b.y, yo) and np.array_equal(b.g, go)
+
+
+@pytest.mark.parametrize("nx,ny", [(1, 1), (5, 6), (29, 64), (43, 44), (44, 44), (61, 64), (90, 90),
+                                   (300, 211)])
+def test_fused_control_at_part_edges(nx, ny):
+    """The kept cells of the fused remesh are counted and written in parts of
+    2048 cells: windows of (nx + 3)(ny + 3) cells around one and several parts
+    give exactly the remesh followed by PopulationControl."""
+    import pfblob
+    rng = np.random.default_rng(100 * nx + ny)
+    h = 0.01
+    X, Y = np.meshgrid((np.arange(nx) + 0.3) * h, (np.arange(ny) + 0.6) * h, indexing="ij")
+    x, y = X.ravel().copy(), Y.ravel().copy()
+    g = np.where(rng.random(x.size) < 0.3, 1.0, 1e-14) * rng.standard_normal(x.size)
+    t = [torch.from_numpy(a).cuda() for a in (x, y, g)]
+    thr = (1e-8, 1e-8)
+    fx, fy, fg, ft = pfblob.remesh_device(*t, h, -1.5 * h, -1.5 * h, population_control=thr)
+    rx, ry, rg = pfblob.remesh_device(*t, h, -1.5 * h, -1.5 * h)
+    px, py, pg, pt = pfblob.population_control_device(rx, ry, rg, *thr)
+    assert torch.equal(fx, px) and torch.equal(fy, py) and torch.equal(fg, pg) and ft == pt
