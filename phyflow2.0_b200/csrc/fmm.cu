@@ -1177,10 +1177,11 @@ static size_t fmm_scratch_bytes(const FmmCache &c, int64_t ns, int64_t nt, bool 
 // ctr: FMM_COUNTERS device counters (P2P pairs, M2L translations, P2P pairs
 // evaluated without the exponential), zeroed here.
 // ev: 7 events recorded around the phases, or nullptr.
+// side: a second stream for the far field, or nullptr (everything on st).
 template <int NP>
 static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, double x0,
                           double y0, double w0, unsigned long long *ctr, cudaEvent_t *ev,
-                          cudaStream_t st) {
+                          const pf::SideStream *side, cudaStream_t st) {
     const int L = c.L, kb = c.kb;
     const bool same = (a.xt == a.x && a.yt == a.y && a.nt == a.ns);
     const double wl = std::ldexp(w0, -L);
@@ -1247,8 +1248,6 @@ static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, dou
         PF_TRY(sort_points(nt, a.xt, a.yt, nullptr, x0, y0, wl, L, T, tmp, tkey_sorted, big + 1,
                            big, st));
     if (same) T = S;  // sort_points replaced S.perm by the final permutation
-    PF_TRY(count_up(L, scnt_all, st));
-    if (!same) PF_TRY(count_up(L, tcnt_all, st));
     // the near field's description
     const int64_t nblk = (int64_t)1 << (2 * (L - kb));
     P2PDesc pd;
@@ -1274,57 +1273,7 @@ static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, dou
     pd.nt = nt;
 
     PF_TRY(mark(1));
-    // upward pass
-    k_p2m<NP><<<(unsigned)pf::ceil_div(4 * nleaf, 128), 128, 0, st>>>(L, x0, y0, wl, S.start, S.cnt,
-                                                                 S.x, S.y, S.g, M);
-    PF_TRY(pf::launch_status("k_p2m"));
-    // parents at levels L-1 .. 2: two levels per launch, one more when odd
-    int lp = L - 1;
-    for (; lp - 1 >= 2; lp -= 2) {
-        const int64_t tasks = ((int64_t)1 << (2 * lp)) / 4;
-        k_m2m_tc<NP><<<(unsigned)pf::ceil_div(tasks, TC_THREADS / 32), TC_THREADS, 0, st>>>(
-            lp, true, scnt_all, M, c.d_m2m);
-        PF_TRY(pf::launch_status("k_m2m_tc"));
-    }
-    if (lp >= 2) {
-        const int64_t tasks = ((int64_t)1 << (2 * lp)) / 4;
-        k_m2m_tc<NP><<<(unsigned)pf::ceil_div(tasks, TC_THREADS / 32), TC_THREADS, 0, st>>>(
-            lp, false, scnt_all, M, c.d_m2m);
-        PF_TRY(pf::launch_status("k_m2m_tc"));
-    }
-    PF_TRY(mark(2));
-    // M2L, all levels >= 2
-    const int B = 1 << kb, Bp = B > 2 ? B : 2;
-    {
-        const int64_t nquad = (nbox - level_off(2)) / 4;  // box quads of levels 2..L
-        if (nquad <= M2L_AHEAD_QUADS && a.nt_beside == 0)
-            k_m2l<NP, true><<<(unsigned)nquad, 32, 0, st>>>(
-                L, Bp, nquad, scnt_all, tcnt_all, M, Lc, c.d_far, c.d_far_ptr, c.maxpos, c.d_pw,
-                c.d_bin, ctr + 1);
-        else
-            k_m2l<NP, false><<<(unsigned)pf::ceil_div(nquad, M2L_THREADS / 32), M2L_THREADS, 0,
-                               st>>>(L, Bp, nquad, scnt_all, tcnt_all, M, Lc, c.d_far,
-                                     c.d_far_ptr, c.maxpos, c.d_pw, c.d_bin, ctr + 1);
-        PF_TRY(pf::launch_status("k_m2l"));
-    }
-    PF_TRY(mark(3));
-    // child levels 3 .. L: two levels per launch, one more when odd
-    int lch = 3;
-    for (; lch + 1 <= L; lch += 2) {
-        const int64_t tasks = ((int64_t)1 << (2 * (lch + 1))) / 16;
-        k_l2l_tc<NP><<<(unsigned)pf::ceil_div(tasks, TC_THREADS / 32), TC_THREADS, 0, st>>>(
-            lch + 1, true, tcnt_all, Lc, c.d_l2l);
-        PF_TRY(pf::launch_status("k_l2l_tc"));
-    }
-    if (lch <= L) {
-        const int64_t tasks = ((int64_t)1 << (2 * lch)) / 16;
-        k_l2l_tc<NP><<<(unsigned)pf::ceil_div(tasks, TC_THREADS / 32), TC_THREADS, 0, st>>>(
-            lch, false, tcnt_all, Lc, c.d_l2l);
-        PF_TRY(pf::launch_status("k_l2l_tc"));
-    }
-    PF_TRY(mark(4));
-    // near field
-    {
+    auto near = [&]() -> pf_status {
         k_p2p_more_groups<<<(unsigned)pf::ceil_div(nblk, 256), 256, 0, st>>>(pd);
         PF_TRY(pf::launch_status("k_p2p_more_groups"));
         const int warps = p2p_warps(nblk, nt, a.nt_beside);
@@ -1334,8 +1283,86 @@ static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, dou
             k_p2p<<<(unsigned)(nblk + p2p_more_ctas(nblk, nt, more_cap)), 32, 0, st>>>(pd);
             PF_TRY(pf::launch_status("k_p2p"));
         }
+        return PF_OK;
+    };
+    auto far = [&](cudaStream_t fs) -> pf_status {
+        // upward pass
+        k_p2m<NP><<<(unsigned)pf::ceil_div(4 * nleaf, 128), 128, 0, fs>>>(L, x0, y0, wl, S.start, S.cnt,
+                                                                     S.x, S.y, S.g, M);
+        PF_TRY(pf::launch_status("k_p2m"));
+        PF_TRY(count_up(L, scnt_all, fs));
+        if (!same) PF_TRY(count_up(L, tcnt_all, fs));
+        // parents at levels L-1 .. 2: two levels per launch, one more when odd
+        int lp = L - 1;
+        for (; lp - 1 >= 2; lp -= 2) {
+            const int64_t tasks = ((int64_t)1 << (2 * lp)) / 4;
+            k_m2m_tc<NP><<<(unsigned)pf::ceil_div(tasks, TC_THREADS / 32), TC_THREADS, 0, fs>>>(
+                lp, true, scnt_all, M, c.d_m2m);
+            PF_TRY(pf::launch_status("k_m2m_tc"));
+        }
+        if (lp >= 2) {
+            const int64_t tasks = ((int64_t)1 << (2 * lp)) / 4;
+            k_m2m_tc<NP><<<(unsigned)pf::ceil_div(tasks, TC_THREADS / 32), TC_THREADS, 0, fs>>>(
+                lp, false, scnt_all, M, c.d_m2m);
+            PF_TRY(pf::launch_status("k_m2m_tc"));
+        }
+        PF_TRY(mark(2));
+        // M2L, all levels >= 2
+        const int B = 1 << kb, Bp = B > 2 ? B : 2;
+        {
+            const int64_t nquad = (nbox - level_off(2)) / 4;  // box quads of levels 2..L
+            if (nquad <= M2L_AHEAD_QUADS && a.nt_beside == 0)
+                k_m2l<NP, true><<<(unsigned)nquad, 32, 0, fs>>>(
+                    L, Bp, nquad, scnt_all, tcnt_all, M, Lc, c.d_far, c.d_far_ptr, c.maxpos, c.d_pw,
+                    c.d_bin, ctr + 1);
+            else
+                k_m2l<NP, false><<<(unsigned)pf::ceil_div(nquad, M2L_THREADS / 32), M2L_THREADS, 0,
+                                   fs>>>(L, Bp, nquad, scnt_all, tcnt_all, M, Lc, c.d_far,
+                                         c.d_far_ptr, c.maxpos, c.d_pw, c.d_bin, ctr + 1);
+            PF_TRY(pf::launch_status("k_m2l"));
+        }
+        PF_TRY(mark(3));
+        // child levels 3 .. L: two levels per launch, one more when odd
+        int lch = 3;
+        for (; lch + 1 <= L; lch += 2) {
+            const int64_t tasks = ((int64_t)1 << (2 * (lch + 1))) / 16;
+            k_l2l_tc<NP><<<(unsigned)pf::ceil_div(tasks, TC_THREADS / 32), TC_THREADS, 0, fs>>>(
+                lch + 1, true, tcnt_all, Lc, c.d_l2l);
+            PF_TRY(pf::launch_status("k_l2l_tc"));
+        }
+        if (lch <= L) {
+            const int64_t tasks = ((int64_t)1 << (2 * lch)) / 16;
+            k_l2l_tc<NP><<<(unsigned)pf::ceil_div(tasks, TC_THREADS / 32), TC_THREADS, 0, fs>>>(
+                lch, false, tcnt_all, Lc, c.d_l2l);
+            PF_TRY(pf::launch_status("k_l2l_tc"));
+        }
+        return PF_OK;
+    };
+    // The near field and the far field (upward pass, M2L, downward pass) share
+    // no data: where the caller gives a second stream (and asks for no phase
+    // events) they run side by side.  Few blobs leave the SMs idle under either
+    // chain; many blobs keep the FP32/exp pipes busy in the one and the FP64
+    // tensor pipe in the other.  Serial -> side by side, uniform blobs: 1,000
+    // 94 -> 83 us, 30,000 197 -> 146, 60,000 222 -> 177, 200,000 426 -> 354,
+    // 500,000 806 -> 714, 2^20 1315 -> 1224; 1.8 million beside a wall
+    // 2431 -> 2272.  The near field is enqueued first: it is the longer chain
+    // (far first: 1,000 95, 60,000 180).  Both statuses are looked at after the
+    // join, so that the caller's stream always waits for the far field.
+    if (side && !ev) {
+        PF_CUDA_TRY(cudaEventRecord(side->fork, st));
+        PF_CUDA_TRY(cudaStreamWaitEvent(side->stream, side->fork, 0));
+        const pf_status sn = near();
+        const pf_status sf = far(side->stream);
+        PF_CUDA_TRY(cudaEventRecord(side->join, side->stream));
+        PF_CUDA_TRY(cudaStreamWaitEvent(st, side->join, 0));
+        PF_TRY(sn);
+        PF_TRY(sf);
+    } else {
+        PF_TRY(far(st));
+        PF_TRY(mark(4));
+        PF_TRY(near());
+        PF_TRY(mark(5));
     }
-    PF_TRY(mark(5));
     k_l2p<NP><<<(unsigned)pf::ceil_div(nt, 256), 256, 0, st>>>(nt, L, x0, y0, wl, T.x, T.y,
                                                                tkey_sorted, Lc, nearv, T.perm,
                                                                a.vx, a.vy);
@@ -1370,13 +1397,14 @@ int fmmx::np_for_tol(double tol) {
 }
 
 pf_status fmm_exec(const FmmCache &c, double x0, double y0, double w0, Bump &sc,
-                   const FmmArgs &a, unsigned long long *ctr, cudaEvent_t *ev, cudaStream_t st) {
+                   const FmmArgs &a, unsigned long long *ctr, cudaEvent_t *ev,
+                   const SideStream *side, cudaStream_t st) {
     switch (c.np) {
-        case 16: return exec_fmm<16>(sc, a, c, x0, y0, w0, ctr, ev, st);
-        case 20: return exec_fmm<20>(sc, a, c, x0, y0, w0, ctr, ev, st);
-        case 24: return exec_fmm<24>(sc, a, c, x0, y0, w0, ctr, ev, st);
-        case 28: return exec_fmm<28>(sc, a, c, x0, y0, w0, ctr, ev, st);
-        case 32: return exec_fmm<32>(sc, a, c, x0, y0, w0, ctr, ev, st);
+        case 16: return exec_fmm<16>(sc, a, c, x0, y0, w0, ctr, ev, side, st);
+        case 20: return exec_fmm<20>(sc, a, c, x0, y0, w0, ctr, ev, side, st);
+        case 24: return exec_fmm<24>(sc, a, c, x0, y0, w0, ctr, ev, side, st);
+        case 28: return exec_fmm<28>(sc, a, c, x0, y0, w0, ctr, ev, side, st);
+        case 32: return exec_fmm<32>(sc, a, c, x0, y0, w0, ctr, ev, side, st);
         default:
             // the plan's coefficient arrays are sized for c.np: never run another size on them
             set_error("FMM: %d expansion terms is not an instantiated size (16, 20, 24, 28, 32)",
@@ -1489,6 +1517,16 @@ extern "C" pf_status pf_fmm_tree_keys(pf_ctx *ctx, int64_t n, const double *x, c
 
 namespace {
 
+// Up to this leaf level the far field runs on a side stream of high priority.
+// Few boxes: the far chain is short kernels in series, each of which should
+// start at once although the near field's CTAs are queued (30,000 blobs 146 us
+// against 156 at the caller's priority, 60,000 beside a wall 160 / 171).  Many
+// boxes: M2L fills the chip, and CTAs let in one by one between the near
+// field's share the SMs' pipes better (500,000 714 us against 747, 2^20 1224 /
+// 1264, 1.8 million beside a wall 2272 / 2350; 200,000, the first size past the
+// line, 354 / 356 uniform, 281 / 275 beside a wall).
+constexpr int SIDE_FIRST_LEVEL = 6;
+
 // pf_velocity_fmm (box == nullptr: bounding box of sources and targets read
 // back from the device, one synchronisation) and pf_velocity_fmm_box (box
 // given by the caller, no synchronisation).
@@ -1588,7 +1626,8 @@ pf_status velocity_fmm(pf_ctx *ctx, int64_t n_src, const double *x, const double
     pf::Bump sc{ctx->arena.base, ctx->arena.cap, 0};
     return pf::fmm_exec(*cache, xmin, ymin, w0, sc, a,
                         reinterpret_cast<unsigned long long *>(ctx->dev_small),
-                        ctx->fmm_profile ? ctx->ev : nullptr, st);
+                        ctx->fmm_profile ? ctx->ev : nullptr,
+                        pf::side_stream(ctx, L <= SIDE_FIRST_LEVEL, st), st);
 }
 
 }  // namespace
@@ -1698,7 +1737,7 @@ pf_status plan_exec(const Plan *p, Bump &sc, int64_t ns, const double *x, const 
                     double ksigmasqr, double *vx, double *vy, int64_t nt_beside,
                     unsigned long long *ctr, cudaEvent_t *ev, cudaStream_t st) {
     FmmArgs a{ns, nt, x, y, g, xt, yt, ksigmasqr, 0.0, 0.0, 0, vx, vy, nt_beside};
-    return fmm_exec(p->c, p->x0, p->y0, p->w0, sc, a, ctr, ev, st);
+    return fmm_exec(p->c, p->x0, p->y0, p->w0, sc, a, ctr, ev, nullptr, st);
 }
 
 void tuning_get(int *leaf_level, int *np, int *kb) {

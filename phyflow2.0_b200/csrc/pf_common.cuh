@@ -89,6 +89,14 @@ struct Arena {
     size_t used = 0;
 };
 
+// A second stream of a context, for work of one call that may run beside the
+// rest: forked from the caller's stream and joined back to it by the events
+// before the call's last kernel, so to the caller the call is on its stream.
+struct SideStream {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+};
+
 }  // namespace pf
 
 struct pf_ctx {
@@ -105,6 +113,8 @@ struct pf_ctx {
     int64_t *dev_small = nullptr;
     bool fmm_profile = false;
     cudaEvent_t ev[8] = {};
+    // [0] the callers' priority, [1] the highest; each created at its first use
+    pf::SideStream side[2];
     cudaStream_t last_stream = nullptr;
     pf_fmm_stats last_stats = {};
     // base cells the remesh scratch is sized for (the last window + 25%)
@@ -129,6 +139,12 @@ struct Bump {
         return p;
     }
 };
+
+// The context's side stream of normal or of the highest priority for work forked
+// from `st` (created on first use), or nullptr where the call has to stay on
+// `st` alone: it can't be created, or it belongs to a capture of another stream.
+const SideStream *side_stream(pf_ctx *ctx, bool first, cudaStream_t st);
+void side_streams_free(pf_ctx *ctx);
 
 // Make sure the arena holds at least `bytes`; may cudaFree/cudaMalloc, which
 // synchronises the device.  Done before any kernel of a call is enqueued.

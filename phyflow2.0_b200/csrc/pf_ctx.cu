@@ -85,6 +85,51 @@ pf_status arena_reserve(pf_ctx *ctx, size_t bytes) {
     return PF_OK;
 }
 
+const SideStream *side_stream(pf_ctx *ctx, bool first, cudaStream_t st) {
+    SideStream &s = ctx->side[first];
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone, ct = cudaStreamCaptureStatusNone;
+    unsigned long long is = 0, it = 0;
+    if (cudaStreamGetCaptureInfo(st, &ct, &it) != cudaSuccess) {
+        cudaGetLastError();  // e.g. the legacy stream while another thread captures
+        return nullptr;
+    }
+    if (!s.stream) {
+        if (ct != cudaStreamCaptureStatusNone) return nullptr;  // nothing is created in a capture
+        int lo = 0, hi = 0;
+        cudaDeviceGetStreamPriorityRange(&lo, &hi);
+        SideStream t;
+        cudaError_t e = cudaStreamCreateWithPriority(&t.stream, cudaStreamNonBlocking,
+                                                     first ? hi : lo);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&t.fork, cudaEventDisableTiming);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&t.join, cudaEventDisableTiming);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            if (t.fork) cudaEventDestroy(t.fork);
+            if (t.stream) cudaStreamDestroy(t.stream);
+            return nullptr;
+        }
+        s = t;
+        return &s;
+    }
+    if (cudaStreamGetCaptureInfo(s.stream, &cs, &is) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    // taken into a capture that is still open: only that capture's stream may use it
+    if (cs != cudaStreamCaptureStatusNone && (cs != ct || is != it)) return nullptr;
+    return &s;
+}
+
+void side_streams_free(pf_ctx *ctx) {
+    for (SideStream &s : ctx->side) {
+        if (!s.stream) continue;
+        cudaEventDestroy(s.fork);
+        cudaEventDestroy(s.join);
+        cudaStreamDestroy(s.stream);
+        s = SideStream{};
+    }
+}
+
 // Readers of the translation units' bounds words (checked build).  A
 // function-local static: units register during library load, in any order.
 static std::vector<BoundsReader> &bounds_readers() {
@@ -163,6 +208,7 @@ pf_status pf_destroy(pf_ctx *ctx) {
     if (ctx->rm_rows) cudaFree(ctx->rm_rows);
     for (int k = 0; k < 8; ++k)
         if (ctx->ev[k]) cudaEventDestroy(ctx->ev[k]);
+    pf::side_streams_free(ctx);
     delete ctx;
     return PF_OK;
 }

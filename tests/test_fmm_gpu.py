@@ -271,3 +271,59 @@ def test_near_field_warps_per_group(n, cluster):
     sub = rng.choice(xt.size, min(xt.size, 1000), replace=False)
     rx, ry = oracle.velocity_direct(x, y, g, 2 * sigma * sigma, xt[sub].copy(), yt[sub].copy())
     assert normwise_err(vx[sub], vy[sub], rx, ry) <= TOL
+
+
+@pytest.mark.parametrize("n", [600, 30000, 140000, 150000])
+@pytest.mark.parametrize("targets", [False, True])
+def test_far_field_beside_near_field(n, targets):
+    """The far field runs on the context's second stream (of high priority up to
+    leaf level 6, reached below about 143,000 blobs; of the caller's beyond):
+    bitwise the phase-timed call, which runs everything on one stream, on the
+    legacy default stream and on others, captured and replayed on new values,
+    and for a call on another stream while such a capture is open."""
+    import pfblob
+    from pfblob import _lib
+    rng = np.random.default_rng(n)
+    x, y = T(rng.random(n)), T(rng.random(n))
+    g = T(rng.standard_normal(n) / n)
+    xt, yt = (T(rng.random(n // 2 + 1)), T(rng.random(n // 2 + 1))) if targets else (x, y)
+    ks, xo, cut = pfblob.fmm_parameters(2.0 / np.sqrt(n))
+    outs = [tuple(torch.full_like(xt, np.nan) for _ in range(2)) for _ in range(5)]
+
+    def call(k, box=(0.0, 1.0, 0.0, 1.0)):
+        pfblob.velocity_device(x, y, g, ks, xt, yt, *outs[k], method=pfblob.FMM_METHOD,
+                               xopt=xo, cutoff=cut, box=box)
+
+    def serial(k):
+        _lib.fmm_profile(True)
+        try:
+            call(k)
+        finally:
+            _lib.fmm_profile(False)
+
+    serial(0)
+    call(1)
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(outs[0], outs[1]))
+    if _lib.CHECKED:
+        return  # the checked build reads its bounds words after each call: no capture
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=s1, capture_error_mode="thread_local"):
+        call(2)
+        with torch.cuda.stream(s2):
+            call(3)
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, b) for a, b in zip(outs[0], outs[3]))
+    g.mul_(-0.75)
+    for v in outs[1]:
+        v.fill_(np.nan)
+    graph.replay()
+    torch.cuda.synchronize()
+    serial(0)
+    torch.cuda.synchronize()  # the calls share their context's scratch
+    with torch.cuda.stream(s2):
+        call(4)
+    torch.cuda.synchronize()
+    for k in (2, 4):
+        assert all(torch.equal(a, b) for a, b in zip(outs[0], outs[k])), k
