@@ -118,76 +118,89 @@ __host__ inline double unord_d(unsigned long long u) {
 
 struct BBox {
     unsigned long long mnx, mxx, mny, mxy;
-    int bad;
-    int pad[7];
+    unsigned long long bad;
 };
 
-__global__ void k_bbox_init(BBox *b) {
-    b->mnx = b->mny = ~0ull;
-    b->mxx = b->mxy = 0ull;
-    b->bad = 0;
+__device__ __forceinline__ void bbox_merge(BBox &a, const BBox &b) {
+    a.mnx = min(a.mnx, b.mnx);
+    a.mxx = max(a.mxx, b.mxx);
+    a.mny = min(a.mny, b.mny);
+    a.mxy = max(a.mxy, b.mxy);
+    a.bad |= b.bad;
 }
 
+// the block's box, valid in thread 0
+__device__ __forceinline__ void bbox_block(BBox &v, BBox *s_v) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        BBox w;
+        w.mnx = __shfl_xor_sync(0xffffffffu, v.mnx, o);
+        w.mxx = __shfl_xor_sync(0xffffffffu, v.mxx, o);
+        w.mny = __shfl_xor_sync(0xffffffffu, v.mny, o);
+        w.mxy = __shfl_xor_sync(0xffffffffu, v.mxy, o);
+        w.bad = 0;
+        bbox_merge(v, w);
+    }
+    v.bad = __reduce_or_sync(0xffffffffu, (unsigned)v.bad);
+    if ((threadIdx.x & 31) == 0) s_v[threadIdx.x >> 5] = v;
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < 8; ++w) bbox_merge(v, s_v[w]);
+}
+
+// Bounding box of n sources and nt targets in one launch: each CTA leaves its
+// box in part[], the last one to finish (ticket, which wraps back to zero)
+// merges them and writes the result to the host's pinned memory, where the
+// caller reads it after the stream's synchronisation.  Latency-bound: a
+// preparing launch, a second launch for separate targets and the copy cost
+// 2-5 us each; with the other launches merged, see k_place, 1,000 blobs
+// 83 -> 65 us, 30,000 146 -> 125 a call.
 __global__ void __launch_bounds__(256)
-k_bbox(const double *__restrict__ x, const double *__restrict__ y, int64_t n, BBox *b) {
-    unsigned long long mnx = ~0ull, mxx = 0, mny = ~0ull, mxy = 0;
-    int bad = 0;
+k_bbox(const double *__restrict__ x, const double *__restrict__ y, int64_t n,
+       const double *__restrict__ xt, const double *__restrict__ yt, int64_t nt, BBox *part,
+       unsigned *ticket, BBox *out) {
+    __shared__ BBox s_v[8];
+    __shared__ bool s_last;
+    BBox v{~0ull, 0, ~0ull, 0, 0};
     // four independent loads of x and y per thread in flight
-    const int64_t stride = (int64_t)gridDim.x * 256;
-    for (int64_t i0 = (int64_t)blockIdx.x * 256 + threadIdx.x; i0 < n; i0 += 4 * stride) {
+    const int64_t stride = (int64_t)gridDim.x * 256, m = n + nt;
+    for (int64_t i0 = (int64_t)blockIdx.x * 256 + threadIdx.x; i0 < m; i0 += 4 * stride) {
         double a[4], c[4];
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
             const int64_t i = i0 + u * stride;
-            a[u] = i < n ? x[i] : 0.0;
-            c[u] = i < n ? y[i] : 0.0;
+            a[u] = i < n ? x[i] : i < m ? xt[i - n] : 0.0;
+            c[u] = i < n ? y[i] : i < m ? yt[i - n] : 0.0;
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
-            if (i0 + u * stride >= n) continue;
+            if (i0 + u * stride >= m) continue;
             if (!isfinite(a[u]) || !isfinite(c[u])) {
-                bad = 1;
+                v.bad = 1;
                 continue;
             }
             const unsigned long long oa = ord_d(a[u]), oc = ord_d(c[u]);
-            mnx = min(mnx, oa);
-            mxx = max(mxx, oa);
-            mny = min(mny, oc);
-            mxy = max(mxy, oc);
+            bbox_merge(v, BBox{oa, oa, oc, oc, 0});
         }
     }
-    for (int o = 16; o; o >>= 1) {
-        mnx = min(mnx, __shfl_xor_sync(0xffffffffu, mnx, o));
-        mxx = max(mxx, __shfl_xor_sync(0xffffffffu, mxx, o));
-        mny = min(mny, __shfl_xor_sync(0xffffffffu, mny, o));
-        mxy = max(mxy, __shfl_xor_sync(0xffffffffu, mxy, o));
-    }
-    bad = __reduce_or_sync(0xffffffffu, bad);
-    // block reduction, then one set of atomics per block
-    __shared__ unsigned long long s_v[4][8];
-    __shared__ int s_bad[8];
-    const int wid = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) {
-        s_v[0][wid] = mnx;
-        s_v[1][wid] = mxx;
-        s_v[2][wid] = mny;
-        s_v[3][wid] = mxy;
-        s_bad[wid] = bad;
+    bbox_block(v, s_v);
+    if (threadIdx.x == 0) {
+        part[blockIdx.x] = v;
+        __threadfence();
+        s_last = atomicInc(ticket, gridDim.x - 1) == gridDim.x - 1;
     }
     __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    v = BBox{~0ull, 0, ~0ull, 0, 0};
+    for (unsigned k = threadIdx.x; k < gridDim.x; k += 256) {
+        const unsigned long long *p = reinterpret_cast<const unsigned long long *>(part + k);
+        bbox_merge(v, BBox{__ldcg(p), __ldcg(p + 1), __ldcg(p + 2), __ldcg(p + 3), __ldcg(p + 4)});
+    }
+    bbox_block(v, s_v);
     if (threadIdx.x == 0) {
-        for (int w = 1; w < 8; ++w) {
-            mnx = min(mnx, s_v[0][w]);
-            mxx = max(mxx, s_v[1][w]);
-            mny = min(mny, s_v[2][w]);
-            mxy = max(mxy, s_v[3][w]);
-            bad |= s_bad[w];
-        }
-        atomicMin(&b->mnx, mnx);
-        atomicMax(&b->mxx, mxx);
-        atomicMin(&b->mny, mny);
-        atomicMax(&b->mxy, mxy);
-        if (bad) atomicOr(&b->bad, 1);
+        *out = v;
+        __threadfence_system();
     }
 }
 
@@ -196,25 +209,17 @@ k_bbox(const double *__restrict__ x, const double *__restrict__ y, int64_t n, BB
 __global__ void __launch_bounds__(256)
 k_leaf_keys(const double *__restrict__ x, const double *__restrict__ y, int64_t n, double x0,
             double y0, double wl, int L, uint32_t *__restrict__ key, int32_t *__restrict__ rank,
-            int32_t *__restrict__ cnt) {
+            int32_t *__restrict__ cnt, int32_t *__restrict__ big_n,
+            unsigned long long *__restrict__ ctr) {
     const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    // the first launch of a call clears its counters: memsets were launches
+    if (i == 0 && big_n) *big_n = 0;
+    if (i == 0 && ctr)
+        for (int k = 0; k < pf::fmmx::FMM_COUNTERS; ++k) ctr[k] = 0;
     if (i >= n) return;
     const uint32_t k = morton2(leaf_coord(x[i], x0, wl, L), leaf_coord(y[i], y0, wl, L));
     key[i] = k;
     if (rank) rank[i] = atomicAdd(&cnt[k], 1);
-}
-
-__global__ void __launch_bounds__(256)
-k_place(int64_t n, const uint32_t *__restrict__ key, const int32_t *__restrict__ rank,
-        const int32_t *__restrict__ start, int32_t *__restrict__ perm, int32_t *__restrict__ big,
-        int32_t *__restrict__ big_n) {
-    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
-    if (i >= n) return;
-    const int64_t p = (int64_t)start[key[i]] + rank[i];
-    if (PF_IDX_OK(p, n, 201)) perm[p] = (int32_t)i;
-    // a leaf of more than LEAF_SMALL particles (exactly one has this rank) is
-    // listed for the segment sort
-    if (rank[i] == LEAF_SMALL) big[atomicAdd(big_n, 1)] = (int32_t)key[i];
 }
 
 __host__ __device__ __forceinline__ int64_t level_off(int l) {
@@ -265,30 +270,32 @@ k_gather_sorted(int64_t n, const int32_t *__restrict__ perm, const uint32_t *__r
     }
 }
 
-// Box counts of nlev (<= 4) coarser levels from level lc: CTA b owns the
+// Box counts of nlev (<= 6) coarser levels from level lc: CTA b owns the
 // 4^nlev level-lc boxes below box b of level lc - nlev (one contiguous Morton
 // range) and sums them up level by level in shared memory (integer sums:
 // exact, any order).
-__global__ void __launch_bounds__(256)
-k_count_up(int lc, int nlev, int32_t *__restrict__ cnt_all) {
-    __shared__ int32_t s_c[256];
+constexpr int COUNT_LEVELS = 6;
+__device__ __forceinline__ void count_up_block(int lc, int nlev, int64_t b,
+                                               int32_t *__restrict__ cnt_all) {
+    __shared__ int32_t s_c[2][1024];
     const int nch = 1 << (2 * nlev);
-    if ((int)threadIdx.x < nch)
-        s_c[threadIdx.x] = cnt_all[level_off(lc) + (int64_t)blockIdx.x * nch + threadIdx.x];
-    __syncthreads();
+    const int32_t *src = cnt_all + level_off(lc) + b * nch;
     for (int j = 1; j <= nlev; ++j) {
         const int np = nch >> (2 * j);
-        int32_t v = 0;
-        if ((int)threadIdx.x < np)
-            v = s_c[4 * threadIdx.x] + s_c[4 * threadIdx.x + 1] + s_c[4 * threadIdx.x + 2] +
-                s_c[4 * threadIdx.x + 3];
-        __syncthreads();
-        if ((int)threadIdx.x < np) {
-            s_c[threadIdx.x] = v;
-            cnt_all[level_off(lc - j) + (int64_t)blockIdx.x * np + threadIdx.x] = v;
+        int32_t *dst = s_c[j & 1];
+        int32_t *all = cnt_all + level_off(lc - j) + b * np;
+        for (int p = threadIdx.x; p < np; p += 256) {
+            const int32_t v = src[4 * p] + src[4 * p + 1] + src[4 * p + 2] + src[4 * p + 3];
+            dst[p] = v;
+            all[p] = v;
         }
         __syncthreads();
+        src = dst;
     }
+}
+
+__global__ void __launch_bounds__(256) k_count_up(int lc, int nlev, int32_t *__restrict__ cnt_all) {
+    count_up_block(lc, nlev, blockIdx.x, cnt_all);
 }
 
 // ---------------------------------------------------------------------------
@@ -795,8 +802,7 @@ k_p2p_runs(int L, int kb, const int2 *__restrict__ q, int nq, int nqp,
 // beside the first groups' instead of after them in one CTA (1.8e6 blobs in an
 // annulus, three groups in each occupied block: P2P 2.34 -> 2.02 ms).  Each
 // group is computed by one CTA, so results do not depend on the list's order.
-__global__ void __launch_bounds__(256) k_p2p_more_groups(const P2PDesc d) {
-    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+__device__ __forceinline__ void list_more_groups(const P2PDesc &d, int64_t i) {
     if (i >= d.nblk) return;
     const int b = d.order[i];
     int t0;
@@ -805,6 +811,33 @@ __global__ void __launch_bounds__(256) k_p2p_more_groups(const P2PDesc d) {
     const int64_t at = atomicAdd(d.nmore, (unsigned)(ngrp - 1));
     for (int g = 1; g < ngrp; ++g)
         if (PF_IDX_OK(at + g - 1, d.more_cap, 207)) d.more[at + g - 1] = make_int2(b, g);
+}
+
+// Second half of the counting sort, and what else needs only the leaf counts
+// and starts, in CTAs after the sort's gn: nc CTAs sum the counts up `nlev`
+// levels from the leaves (L), the rest list the P2P groups beyond each block's
+// first (d.nblk = 0: none).  As launches of their own the two cost 2-4 us each
+// with their gaps.
+__global__ void __launch_bounds__(256)
+k_place(int64_t n, const uint32_t *__restrict__ key, const int32_t *__restrict__ rank,
+        const int32_t *__restrict__ start, int32_t *__restrict__ perm, int32_t *__restrict__ big,
+        int32_t *__restrict__ big_n, unsigned gn, int L, int nlev, unsigned nc, int32_t *cnt_all,
+        const P2PDesc d) {
+    if (blockIdx.x >= gn + nc) {
+        list_more_groups(d, (int64_t)(blockIdx.x - gn - nc) * 256 + threadIdx.x);
+        return;
+    }
+    if (blockIdx.x >= gn) {
+        count_up_block(L, nlev, blockIdx.x - gn, cnt_all);
+        return;
+    }
+    const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    const int64_t p = (int64_t)start[key[i]] + rank[i];
+    if (PF_IDX_OK(p, n, 201)) perm[p] = (int32_t)i;
+    // a leaf of more than LEAF_SMALL particles (exactly one has this rank) is
+    // listed for the segment sort
+    if (rank[i] == LEAF_SMALL) big[atomicAdd(big_n, 1)] = (int32_t)key[i];
 }
 
 // One CTA (one warp) per target group: CTA i < nblk the first group of block i
@@ -1082,22 +1115,25 @@ struct Sorted {
     float *g32 = nullptr;
 };
 
+// Sort by leaf; also the box counts of all levels (cnt_all, s.cnt its leaf
+// level) up to COUNT_LEVELS above the leaves, see count_up, and with pd.nblk > 0
+// the list of P2P groups.  ctr: the call's counters to clear, or nullptr.  n > 0.
 static pf_status sort_points(int64_t n, const double *x, const double *y,
                              const double *g, double x0, double y0, double wl, int L, Sorted &s,
                              int32_t *scan_tmp, uint32_t *skey, int32_t *big, int32_t *big_n,
+                             int32_t *cnt_all, unsigned long long *ctr, const P2PDesc &pd,
                              cudaStream_t st) {
     const int64_t nleaf = (int64_t)1 << (2 * L);
     PF_CUDA_TRY(cudaMemsetAsync(s.cnt, 0, sizeof(int32_t) * nleaf, st));
-    if (n == 0) {
-        PF_CUDA_TRY(cudaMemsetAsync(s.start, 0, sizeof(int32_t) * nleaf, st));
-        return PF_OK;
-    }
     const unsigned gn = (unsigned)pf::ceil_div(n, 256);
-    k_leaf_keys<<<gn, 256, 0, st>>>(x, y, n, x0, y0, wl, L, s.key, s.rank, s.cnt);
+    k_leaf_keys<<<gn, 256, 0, st>>>(x, y, n, x0, y0, wl, L, s.key, s.rank, s.cnt, big_n, ctr);
     PF_TRY(pf::launch_status("k_leaf_keys"));
     PF_TRY(pf::exclusive_scan_i32(s.cnt, s.start, nleaf, scan_tmp, nullptr, st));
-    PF_CUDA_TRY(cudaMemsetAsync(big_n, 0, sizeof(int32_t), st));
-    k_place<<<gn, 256, 0, st>>>(n, s.key, s.rank, s.start, s.perm, big, big_n);
+    const int nlev = std::min(L, COUNT_LEVELS);
+    const unsigned nc = 1u << (2 * (L - nlev));
+    const unsigned nm = (unsigned)pf::ceil_div(pd.nblk, 256);
+    k_place<<<gn + nc + nm, 256, 0, st>>>(n, s.key, s.rank, s.start, s.perm, big, big_n, gn, L,
+                                          nlev, nc, cnt_all, pd);
     PF_TRY(pf::launch_status("k_place"));
     // leaves above LEAF_SMALL particles (dense clusters); the ranks are free now
     PF_TRY(pf::seg_sort_listed(big, big_n, s.start, s.cnt, s.perm, s.rank,
@@ -1109,15 +1145,12 @@ static pf_status sort_points(int64_t n, const double *x, const double *y,
     return pf::launch_status("k_gather_sorted");
 }
 
+// the box counts of the levels above those that sort_points sums up
 static pf_status count_up(int L, int32_t *cnt_all, cudaStream_t st) {
-    for (int lc = L; lc > 0;) {
-        const int nlev = lc < 4 ? lc : 4;
-        const int64_t nblk = (int64_t)1 << (2 * (lc - nlev));
-        k_count_up<<<(unsigned)nblk, 256, 0, st>>>(lc, nlev, cnt_all);
-        PF_TRY(pf::launch_status("k_count_up"));
-        lc -= nlev;
-    }
-    return PF_OK;
+    static_assert(pf::fmmx::MAX_LEVEL <= 2 * COUNT_LEVELS, "two passes reach the root");
+    if (L <= COUNT_LEVELS) return PF_OK;
+    k_count_up<<<1, 256, 0, st>>>(L - COUNT_LEVELS, L - COUNT_LEVELS, cnt_all);
+    return pf::launch_status("k_count_up");
 }
 
 struct FmmArgs {
@@ -1234,20 +1267,6 @@ static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, dou
         T.start = tstart;
     }
 
-    PF_CUDA_TRY(cudaMemsetAsync(ctr, 0, pf::fmmx::FMM_COUNTERS * sizeof(unsigned long long), st));
-    auto mark = [&](int k) -> pf_status {
-        if (ev) PF_CUDA_TRY(cudaEventRecord(ev[k], st));
-        return PF_OK;
-    };
-    PF_TRY(mark(0));
-    // sort sources (and targets)
-    // sorted target keys come out of the sorted copies of the targets
-    PF_TRY(sort_points(ns, a.x, a.y, a.g, x0, y0, wl, L, S, tmp, same ? tkey_sorted : nullptr,
-                       big + 1, big, st));
-    if (!same)
-        PF_TRY(sort_points(nt, a.xt, a.yt, nullptr, x0, y0, wl, L, T, tmp, tkey_sorted, big + 1,
-                           big, st));
-    if (same) T = S;  // sort_points replaced S.perm by the final permutation
     // the near field's description
     const int64_t nblk = (int64_t)1 << (2 * (L - kb));
     P2PDesc pd;
@@ -1272,11 +1291,25 @@ static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, dou
     pd.ns = ns;
     pd.nt = nt;
 
+    auto mark = [&](int k) -> pf_status {
+        if (ev) PF_CUDA_TRY(cudaEventRecord(ev[k], st));
+        return PF_OK;
+    };
+    PF_TRY(mark(0));
+    // sort sources (and targets)
+    // sorted target keys come out of the sorted copies of the targets
+    P2PDesc none = pd;
+    none.nblk = 0;
+    PF_TRY(sort_points(ns, a.x, a.y, a.g, x0, y0, wl, L, S, tmp, same ? tkey_sorted : nullptr,
+                       big + 1, big, scnt_all, ctr, same ? pd : none, st));
+    if (!same)
+        PF_TRY(sort_points(nt, a.xt, a.yt, nullptr, x0, y0, wl, L, T, tmp, tkey_sorted, big + 1,
+                           big, tcnt_all, nullptr, pd, st));
+    if (same) T = S;  // sort_points replaced S.perm by the final permutation
+
     PF_TRY(mark(1));
+    const int warps = p2p_warps(nblk, nt, a.nt_beside);
     auto near = [&]() -> pf_status {
-        k_p2p_more_groups<<<(unsigned)pf::ceil_div(nblk, 256), 256, 0, st>>>(pd);
-        PF_TRY(pf::launch_status("k_p2p_more_groups"));
-        const int warps = p2p_warps(nblk, nt, a.nt_beside);
         if (warps > 1) {
             PF_TRY(pf::fmmx::launch_p2p_multi(pd, warps, (unsigned)(nblk + more_cap), st));
         } else {
@@ -1342,17 +1375,27 @@ static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, dou
     // no data: where the caller gives a second stream (and asks for no phase
     // events) they run side by side.  Few blobs leave the SMs idle under either
     // chain; many blobs keep the FP32/exp pipes busy in the one and the FP64
-    // tensor pipe in the other.  Serial -> side by side, uniform blobs: 1,000
-    // 94 -> 83 us, 30,000 197 -> 146, 60,000 222 -> 177, 200,000 426 -> 354,
-    // 500,000 806 -> 714, 2^20 1315 -> 1224; 1.8 million beside a wall
-    // 2431 -> 2272.  The near field is enqueued first: it is the longer chain
-    // (far first: 1,000 95, 60,000 180).  Both statuses are looked at after the
-    // join, so that the caller's stream always waits for the far field.
+    // tensor pipe in the other.  Serial -> side by side, uniform blobs: 30,000
+    // 197 -> 157 us, 60,000 222 -> 183, 200,000 426 -> 354, 500,000 806 -> 714,
+    // 2^20 1315 -> 1224; 1.8 million beside a wall 2431 -> 2272.  Several warps per
+    // group, so few groups: the near field is the longer chain and is enqueued
+    // first (12,000 blobs 102 us, far first 106; 30,000 130 / 136).  One warp per
+    // group: its CTAs take all registers of the SMs, and what is enqueued after
+    // them waits for a CTA to end, so the far field goes first (the other way
+    // round with the far field on a stream of high priority, 120,000 326 / 270).
+    // The two streams have the same priority: high priority for the far field
+    // gained 4-5% at 30,000-60,000 blobs, but while a process has streams of two
+    // priorities its batch graphs run 3% slower (12 sets 1337 -> 1372).  Both
+    // statuses are looked at after the join, so that the caller's stream always
+    // waits for the far field.
     if (side && !ev) {
         PF_CUDA_TRY(cudaEventRecord(side->fork, st));
         PF_CUDA_TRY(cudaStreamWaitEvent(side->stream, side->fork, 0));
-        const pf_status sn = near();
+        const bool near_first = warps > 1;
+        pf_status sn = PF_OK;
+        if (near_first) sn = near();
         const pf_status sf = far(side->stream);
+        if (!near_first) sn = near();
         PF_CUDA_TRY(cudaEventRecord(side->join, side->stream));
         PF_CUDA_TRY(cudaStreamWaitEvent(st, side->join, 0));
         PF_TRY(sn);
@@ -1511,21 +1554,12 @@ extern "C" pf_status pf_fmm_tree_keys(pf_ctx *ctx, int64_t n, const double *x, c
     if (n == 0) return PF_OK;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     k_leaf_keys<<<(unsigned)pf::ceil_div(n, 256), 256, 0, st>>>(x, y, n, x0, y0, leaf_width,
-                                                               leaf_level, keys, nullptr, nullptr);
+                                                               leaf_level, keys, nullptr, nullptr,
+                                                               nullptr, nullptr);
     return pf::launch_status("k_leaf_keys");
 }
 
 namespace {
-
-// Up to this leaf level the far field runs on a side stream of high priority.
-// Few boxes: the far chain is short kernels in series, each of which should
-// start at once although the near field's CTAs are queued (30,000 blobs 146 us
-// against 156 at the caller's priority, 60,000 beside a wall 160 / 171).  Many
-// boxes: M2L fills the chip, and CTAs let in one by one between the near
-// field's share the SMs' pipes better (500,000 714 us against 747, 2^20 1224 /
-// 1264, 1.8 million beside a wall 2272 / 2350; 200,000, the first size past the
-// line, 354 / 356 uniform, 281 / 275 beside a wall).
-constexpr int SIDE_FIRST_LEVEL = 6;
 
 // pf_velocity_fmm (box == nullptr: bounding box of sources and targets read
 // back from the device, one synchronisation) and pf_velocity_fmm_box (box
@@ -1577,22 +1611,17 @@ pf_status velocity_fmm(pf_ctx *ctx, int64_t n_src, const double *x, const double
         ymin = box[2];
         ymax = box[3];
     } else {
-        PF_TRY(pf::arena_reserve(ctx, 4096));
-        BBox *bb = static_cast<BBox *>(pf::arena_take(ctx, sizeof(BBox)));
-        k_bbox_init<<<1, 1, 0, st>>>(bb);
-        PF_TRY(pf::launch_status("k_bbox_init"));
-        const int cap = ctx->num_sms * 4;  // each CTA ends in five atomics on the same words
-        k_bbox<<<(unsigned)std::min<int64_t>(pf::ceil_div(n_src, 256), cap), 256, 0, st>>>(
-            x, y, n_src, bb);
+        const int cap = ctx->num_sms * 4;  // each CTA ends in an atomic on the ticket
+        PF_TRY(pf::arena_reserve(ctx, pf::align256(cap * sizeof(BBox))));
+        BBox *part = static_cast<BBox *>(pf::arena_take(ctx, cap * sizeof(BBox)));
+        const int64_t nt_box = (xt == x && yt == y) ? 0 : n_tgt;
+        const int64_t nb = std::min<int64_t>(pf::ceil_div(n_src + nt_box, 256), cap);
+        k_bbox<<<(unsigned)nb, 256, 0, st>>>(
+            x, y, n_src, xt, yt, nt_box, part,
+            reinterpret_cast<unsigned *>(ctx->dev_small + pf::fmmx::FMM_COUNTERS),
+            reinterpret_cast<BBox *>(ctx->host_small));
         PF_TRY(pf::launch_status("k_bbox"));
-        if (!(xt == x && yt == y)) {
-            k_bbox<<<(unsigned)std::min<int64_t>(pf::ceil_div(n_tgt, 256), cap), 256, 0, st>>>(
-                xt, yt, n_tgt, bb);
-            PF_TRY(pf::launch_status("k_bbox"));
-        }
         BBox hb;
-        PF_CUDA_TRY(
-            cudaMemcpyAsync(ctx->host_small, bb, sizeof(BBox), cudaMemcpyDeviceToHost, st));
         PF_CUDA_TRY(cudaStreamSynchronize(st));
         memcpy(&hb, ctx->host_small, sizeof(BBox));
         if (hb.bad) {
@@ -1627,7 +1656,7 @@ pf_status velocity_fmm(pf_ctx *ctx, int64_t n_src, const double *x, const double
     return pf::fmm_exec(*cache, xmin, ymin, w0, sc, a,
                         reinterpret_cast<unsigned long long *>(ctx->dev_small),
                         ctx->fmm_profile ? ctx->ev : nullptr,
-                        pf::side_stream(ctx, L <= SIDE_FIRST_LEVEL, st), st);
+                        pf::side_stream(ctx, st), st);
 }
 
 }  // namespace

@@ -113,8 +113,7 @@ struct pf_ctx {
     int64_t *dev_small = nullptr;
     bool fmm_profile = false;
     cudaEvent_t ev[8] = {};
-    // [0] the callers' priority, [1] the highest; each created at its first use
-    pf::SideStream side[2];
+    pf::SideStream side;  // created at its first use
     cudaStream_t last_stream = nullptr;
     pf_fmm_stats last_stats = {};
     // base cells the remesh scratch is sized for (the last window + 25%)
@@ -140,11 +139,11 @@ struct Bump {
     }
 };
 
-// The context's side stream of normal or of the highest priority for work forked
-// from `st` (created on first use), or nullptr where the call has to stay on
-// `st` alone: it can't be created, or it belongs to a capture of another stream.
-const SideStream *side_stream(pf_ctx *ctx, bool first, cudaStream_t st);
-void side_streams_free(pf_ctx *ctx);
+// The context's side stream for work forked from `st` (created on first use), or
+// nullptr where the call has to stay on `st` alone: it can't be created, or it
+// belongs to a capture of another stream.
+const SideStream *side_stream(pf_ctx *ctx, cudaStream_t st);
+void side_stream_free(pf_ctx *ctx);
 
 // Make sure the arena holds at least `bytes`; may cudaFree/cudaMalloc, which
 // synchronises the device.  Done before any kernel of a call is enqueued.

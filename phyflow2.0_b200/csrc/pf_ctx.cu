@@ -85,8 +85,8 @@ pf_status arena_reserve(pf_ctx *ctx, size_t bytes) {
     return PF_OK;
 }
 
-const SideStream *side_stream(pf_ctx *ctx, bool first, cudaStream_t st) {
-    SideStream &s = ctx->side[first];
+const SideStream *side_stream(pf_ctx *ctx, cudaStream_t st) {
+    SideStream &s = ctx->side;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone, ct = cudaStreamCaptureStatusNone;
     unsigned long long is = 0, it = 0;
     if (cudaStreamGetCaptureInfo(st, &ct, &it) != cudaSuccess) {
@@ -95,11 +95,8 @@ const SideStream *side_stream(pf_ctx *ctx, bool first, cudaStream_t st) {
     }
     if (!s.stream) {
         if (ct != cudaStreamCaptureStatusNone) return nullptr;  // nothing is created in a capture
-        int lo = 0, hi = 0;
-        cudaDeviceGetStreamPriorityRange(&lo, &hi);
         SideStream t;
-        cudaError_t e = cudaStreamCreateWithPriority(&t.stream, cudaStreamNonBlocking,
-                                                     first ? hi : lo);
+        cudaError_t e = cudaStreamCreateWithFlags(&t.stream, cudaStreamNonBlocking);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&t.fork, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&t.join, cudaEventDisableTiming);
         if (e != cudaSuccess) {
@@ -120,14 +117,13 @@ const SideStream *side_stream(pf_ctx *ctx, bool first, cudaStream_t st) {
     return &s;
 }
 
-void side_streams_free(pf_ctx *ctx) {
-    for (SideStream &s : ctx->side) {
-        if (!s.stream) continue;
-        cudaEventDestroy(s.fork);
-        cudaEventDestroy(s.join);
-        cudaStreamDestroy(s.stream);
-        s = SideStream{};
-    }
+void side_stream_free(pf_ctx *ctx) {
+    SideStream &s = ctx->side;
+    if (!s.stream) return;
+    cudaEventDestroy(s.fork);
+    cudaEventDestroy(s.join);
+    cudaStreamDestroy(s.stream);
+    s = SideStream{};
 }
 
 // Readers of the translation units' bounds words (checked build).  A
@@ -192,6 +188,7 @@ pf_status pf_create(int device, pf_ctx **out) {
         return PF_ERR_CUDA;
     }
     cudaMemset(c->dev_small, 0, 4096);
+    cudaStreamSynchronize(cudaStreamLegacy);  // before any other stream's kernel uses it
     *out = c;
     return PF_OK;
 }
@@ -208,7 +205,7 @@ pf_status pf_destroy(pf_ctx *ctx) {
     if (ctx->rm_rows) cudaFree(ctx->rm_rows);
     for (int k = 0; k < 8; ++k)
         if (ctx->ev[k]) cudaEventDestroy(ctx->ev[k]);
-    pf::side_streams_free(ctx);
+    pf::side_stream_free(ctx);
     delete ctx;
     return PF_OK;
 }

@@ -1,5 +1,5 @@
-// scan.cu -- three-pass exclusive scan: per-tile scan + tile totals, one-block
-// scan of the totals, add the tile offsets.  Warp-shuffle inclusive scans
+// scan.cu -- exclusive scan: per-tile scan + tile totals, then each tile adds the
+// totals before it (one tile: one launch).  Warp-shuffle inclusive scans
 // inside each tile; SCAN_ITEMS consecutive elements per thread (coalesced as
 // int4).  Deterministic (integer).
 #include "scan.cuh"
@@ -42,7 +42,7 @@ __device__ __forceinline__ int block_excl_scan(int v, int *s_warp, int *total) {
 
 __global__ void __launch_bounds__(SCAN_THREADS)
 k_scan_tiles(const int32_t *__restrict__ in, int32_t *__restrict__ out, int64_t len,
-             int32_t *__restrict__ tile_tot) {
+             int32_t *__restrict__ tile_tot, int32_t *__restrict__ total_dev) {
     __shared__ int s_warp[33];
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
     int v[SCAN_ITEMS];
@@ -59,7 +59,10 @@ k_scan_tiles(const int32_t *__restrict__ in, int32_t *__restrict__ out, int64_t 
         if (base + k < len) out[base + k] = ex;
         ex += v[k];
     }
-    if (threadIdx.x == 0) tile_tot[blockIdx.x] = tot;
+    if (threadIdx.x == 0) {
+        tile_tot[blockIdx.x] = tot;
+        if (gridDim.x == 1 && total_dev) *total_dev = tot;
+    }
 }
 
 __global__ void __launch_bounds__(SCAN_THREADS)
@@ -77,10 +80,23 @@ k_scan_totals(int32_t *__restrict__ tot, int64_t ntiles, int32_t *__restrict__ t
     if (threadIdx.x == 0 && total_dev) *total_dev = carry;
 }
 
+// tile_off: the tiles' offsets (k_scan_totals), or with tot set their totals,
+// which each CTA sums up to its own tile itself.
 __global__ void __launch_bounds__(SCAN_THREADS)
-k_scan_add(int32_t *__restrict__ out, int64_t len, const int32_t *__restrict__ tile_off) {
+k_scan_add(int32_t *__restrict__ out, int64_t len, const int32_t *__restrict__ tile_off, bool tot,
+           int32_t *__restrict__ total_dev) {
     const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + (int64_t)threadIdx.x * SCAN_ITEMS;
-    const int off = tile_off[blockIdx.x];
+    __shared__ int s_warp[33];
+    int off;
+    if (tot) {
+        int s = 0;
+        for (unsigned i = threadIdx.x; i < blockIdx.x; i += SCAN_THREADS) s += tile_off[i];
+        block_excl_scan(s, s_warp, &off);
+        if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0 && total_dev)
+            *total_dev = off + tile_off[blockIdx.x];
+    } else {
+        off = tile_off[blockIdx.x];
+    }
     if (off == 0) return;
 #pragma unroll
     for (int k = 0; k < SCAN_ITEMS; ++k)
@@ -88,6 +104,11 @@ k_scan_add(int32_t *__restrict__ out, int64_t len, const int32_t *__restrict__ t
 }
 
 }  // namespace
+
+// Up to this many tiles each CTA of the last pass sums the totals before its
+// own tile (at most 8 loads a thread, 33 million elements), beyond it one CTA
+// scans them in a launch of its own, 2 us and a gap of 2 us.
+constexpr int64_t SCAN_SELF_TILES = 8 * SCAN_THREADS;
 
 namespace pf {
 
@@ -102,15 +123,16 @@ pf_status exclusive_scan_i32(const int32_t *in, int32_t *out, int64_t len, int32
         set_error("exclusive_scan_i32: length %lld too large", (long long)len);
         return PF_ERR_INVALID_ARG;
     }
-    k_scan_tiles<<<(unsigned)ntiles, SCAN_THREADS, 0, st>>>(in, out, len, tmp);
+    k_scan_tiles<<<(unsigned)ntiles, SCAN_THREADS, 0, st>>>(in, out, len, tmp, total_dev);
     PF_TRY(launch_status("k_scan_tiles"));
-    k_scan_totals<<<1, SCAN_THREADS, 0, st>>>(tmp, ntiles, total_dev);
-    PF_TRY(launch_status("k_scan_totals"));
-    if (ntiles > 1) {
-        k_scan_add<<<(unsigned)ntiles, SCAN_THREADS, 0, st>>>(out, len, tmp);
-        PF_TRY(launch_status("k_scan_add"));
+    if (ntiles == 1) return PF_OK;
+    const bool self = ntiles <= SCAN_SELF_TILES;
+    if (!self) {
+        k_scan_totals<<<1, SCAN_THREADS, 0, st>>>(tmp, ntiles, total_dev);
+        PF_TRY(launch_status("k_scan_totals"));
     }
-    return PF_OK;
+    k_scan_add<<<(unsigned)ntiles, SCAN_THREADS, 0, st>>>(out, len, tmp, self, total_dev);
+    return launch_status("k_scan_add");
 }
 
 }  // namespace pf

@@ -1,4 +1,4 @@
-// scan.cuh -- device-wide exclusive prefix sum of int32 counts (3 passes).
+// scan.cuh -- device-wide exclusive prefix sum of int32 counts (1 to 3 launches).
 #pragma once
 #include "pf_common.cuh"
 

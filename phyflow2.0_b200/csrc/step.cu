@@ -92,7 +92,7 @@ extern "C" pf_status pf_step_graph_create(pf_ctx *ctx, const pf_step *s, pf_step
         g->graph = gr;
         if (st == PF_OK) e = e2;
     }
-    pf::side_streams_free(g->ctx);  // the graph keeps the fork, not the stream
+    pf::side_stream_free(g->ctx);  // the graph keeps the fork, not the stream
     if (st == PF_OK && e == cudaSuccess) e = cudaGraphInstantiate(&g->exec, g->graph, 0);
     if (st == PF_OK && e == cudaSuccess) e = pf::graph_kernel_nodes(g->graph, &g->kernels);
     if (st != PF_OK || e != cudaSuccess) {

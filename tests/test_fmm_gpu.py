@@ -276,9 +276,8 @@ def test_near_field_warps_per_group(n, cluster):
 @pytest.mark.parametrize("n", [600, 30000, 140000, 150000])
 @pytest.mark.parametrize("targets", [False, True])
 def test_far_field_beside_near_field(n, targets):
-    """The far field runs on the context's second stream (of high priority up to
-    leaf level 6, reached below about 143,000 blobs; of the caller's beyond):
-    bitwise the phase-timed call, which runs everything on one stream, on the
+    """The far field runs on the context's second stream, enqueued before or after
+    the near field by the near field's warps per group: bitwise the phase-timed call, which runs everything on one stream, on the
     legacy default stream and on others, captured and replayed on new values,
     and for a call on another stream while such a capture is open."""
     import pfblob
@@ -327,3 +326,43 @@ def test_far_field_beside_near_field(n, targets):
     torch.cuda.synchronize()
     for k in (2, 4):
         assert all(torch.equal(a, b) for a, b in zip(outs[0], outs[k])), k
+
+
+@pytest.mark.parametrize("leaf_level", [3, 6, 7, 9, 11])
+@pytest.mark.parametrize("n,nt", [(1, 1), (255, 257), (6000, 3000)])
+def test_tree_of_every_leaf_level(leaf_level, n, nt):
+    """The leaf scan (one tile up to level 6, self-summed tiles beyond), the box
+    counts summed up beside the sort (6 levels, a second pass beyond) and the one
+    launch over sources and separate targets for the bounding box: blobs of one
+    sign, targets outside the sources' box too, against the oracle; bitwise the
+    call that is given the exact box; NaN and Inf in the targets refused."""
+    import pfblob
+    from pfblob import _lib
+    rng = np.random.default_rng(31 * n + leaf_level)
+    x, y = rng.random(n), rng.random(n)
+    xt, yt = 3.0 * rng.random(nt) - 1.0, 2.0 * rng.random(nt) - 0.5
+    g = (0.5 + rng.random(n)) / n
+    sigma = 1e-3
+    ks, xo, cut = pfblob.fmm_parameters(sigma)
+    xa, ya = np.append(x, xt), np.append(y, yt)
+    box = (xa.min(), xa.max(), ya.min(), ya.max())
+    # one blob or target alone would take the direct sum: the level is forced
+    _lib.fmm_set_tuning(leaf_level, 0, 1)
+    try:
+        out = []
+        for b in (None, box):
+            v = [torch.empty(nt, dtype=torch.float64, device=DEV) for _ in range(2)]
+            pfblob.velocity_device(T(x), T(y), T(g), ks, T(xt), T(yt), *v,
+                                   method=pfblob.FMM_METHOD, xopt=xo, cutoff=cut, box=b)
+            out.append([a.cpu().numpy() for a in v])
+        assert _lib.fmm_last_stats(DEV.index)["leaf_level"] == leaf_level
+        for bad in (np.nan, np.inf):
+            xb = xt.copy()
+            xb[-1] = bad
+            with pytest.raises(_lib.PfError):
+                fmm(x, y, g, sigma, xt=xb, yt=yt)
+    finally:
+        _lib.fmm_set_tuning(0, 0, 1)
+    assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
+    rx, ry = oracle.velocity_direct(x, y, g, 2 * sigma * sigma, xt, yt)
+    assert normwise_err(*out[0], rx, ry) <= TOL
