@@ -7,8 +7,8 @@
 //   * instances using the direct sum are evaluated together by ONE persistent
 //     kernel that takes (instance, target tile) items from a device counter,
 //     largest first (k_direct_batch);
-//   * FMM instances and all remesh jobs are spread over library streams
-//     (longest-processing-time-first by estimated cost), fork/joined inside
+//   * FMM instances and remesh jobs are spread over library streams of their
+//     own (longest-processing-time-first by estimated time), fork/joined inside
 //     the capture, so independent instances overlap on the GPU;
 //   * nothing in the graph synchronises with the host or allocates.
 // pf_batch_run replays the graph with a single launch.  The reference has no
@@ -40,6 +40,13 @@ struct Job {
     size_t scratch;
 };
 
+// Time of a job alone on the device (us), for their distribution: both have a
+// part that does not depend on the size, their ~15 or ~10 kernels in series.
+double fmm_job_us(int64_t n, int np) {
+    return 80.0 + 2e-3 * (double)n * (np * np / 256.0 + 30.0) / 31.0;
+}
+double remesh_job_us(int64_t n) { return 32.0 + 1.3e-4 * (double)n; }
+
 // host copy of the remesh window-left index (same operation order as the device)
 int64_t left_index_host(double x, double b0, double h) {
     const double h2 = 2.0 * h, h05 = 0.5 * h;
@@ -61,7 +68,7 @@ struct pf_batch {
     std::vector<pf::fmmx::Plan *> plans;
     std::vector<int> method;  // resolved
     std::vector<int64_t> ixmin, iymin, nbx, nby;
-    int nstreams = 0;
+    int nstreams = 0;  // as asked for, then with the remeshes' slots
     std::vector<cudaStream_t> streams;
     cudaStream_t direct_stream = nullptr, cap_stream = nullptr;
     std::vector<cudaEvent_t> events;
@@ -85,15 +92,25 @@ struct pf_batch {
     int64_t n_direct = 0, n_fmm = 0;
 };
 
+// What only the capture needs
+static void batch_free_streams(pf_batch *b) {
+    for (auto s : b->streams)
+        if (s) cudaStreamDestroy(s);
+    b->streams.clear();
+    if (b->direct_stream) cudaStreamDestroy(b->direct_stream);
+    if (b->cap_stream) cudaStreamDestroy(b->cap_stream);
+    b->direct_stream = b->cap_stream = nullptr;
+    for (auto e : b->events)
+        if (e) cudaEventDestroy(e);
+    b->events.clear();
+}
+
 static void batch_free(pf_batch *b) {
     if (!b) return;
     if (b->exec) cudaGraphExecDestroy(b->exec);
     if (b->graph) cudaGraphDestroy(b->graph);
     for (auto *p : b->plans) pf::fmmx::plan_free(p);
-    for (auto s : b->streams) cudaStreamDestroy(s);
-    if (b->direct_stream) cudaStreamDestroy(b->direct_stream);
-    if (b->cap_stream) cudaStreamDestroy(b->cap_stream);
-    for (auto e : b->events) cudaEventDestroy(e);
+    batch_free_streams(b);
     for (auto p : b->slot_scratch) cudaFree(p);
     cudaFree(b->d_ctr);
     cudaFree(b->d_dinst);
@@ -145,7 +162,7 @@ static pf_status batch_build(pf_batch *b, double tol) {
             if (L >= 3) {
                 b->plans[i] = p;
                 m = PF_FMM_METHOD;
-                jobs.push_back({i, 0, (double)d.n * (np * np / 256.0 + 30.0),
+                jobs.push_back({i, 0, fmm_job_us(d.n, np),
                                 pf::fmmx::plan_scratch(p, d.n, d.n, true)});
                 ++b->n_fmm;
             } else {
@@ -191,7 +208,7 @@ static pf_status batch_build(pf_batch *b, double tol) {
                 pf::set_error("pf_batch_create: instance %d remesh window invalid", i);
                 return PF_ERR_INVALID_ARG;
             }
-            jobs.push_back({i, 1, 0.05 * (double)d.n,
+            jobs.push_back({i, 1, remesh_job_us(d.n),
                             pf::remesh_scratch_bytes(d.n, b->nbx[i] * b->nby[i],
                                                      (b->nbx[i] + 3) * (b->nby[i] + 3), false) +
                                 1024});
@@ -225,14 +242,28 @@ static pf_status batch_build(pf_batch *b, double tol) {
         PF_CUDA_TRY(cudaMalloc(&b->d_counter, 16));
         b->direct_grid = pf::direct_batch_grid(ctx->num_sms);
     }
-    // longest processing time first onto the streams
+    // Longest processing time first: FMM jobs onto n_streams slots, remeshes onto
+    // as many others (they read the same inputs as the velocity, not its result).
+    // On one stream each remesh is ten small kernels in series, 30-40 us, which
+    // start late behind the FMM's large grids; shared slots put them all behind
+    // one set's velocity.  12 sets of 2,048 to 131,072 blobs: all remeshes in one
+    // slot 1340-1375 us (what a cost by size alone gives), spread over the FMM's
+    // slots by time 1175, before the FMM in each of them 1117-1132, slots of their
+    // own 1 / 2 / 4 / 8: 1334-1370 / 1190 / 1111 / 1105.  One stream asked for: one
+    // job at a time.
     std::stable_sort(jobs.begin(), jobs.end(),
                      [](const Job &a, const Job &c) { return a.cost > c.cost; });
-    const int S = b->nstreams;
+    int64_t n_rm = 0;
+    for (const Job &j : jobs) n_rm += j.kind == 1;
+    const int F = b->nstreams, S = F > 1 ? F + (int)std::min<int64_t>(n_rm, F) : F;
+    b->nstreams = S;
     b->slot_jobs.assign(S, {});
     std::vector<double> load(S, 0.0);
     for (const Job &j : jobs) {
-        const int s = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+        const bool own = j.kind == 1 && S > F;
+        const auto lo = load.begin() + (own ? F : 0);
+        const auto hi = own ? load.end() : load.begin() + F;
+        const int s = (int)(std::min_element(lo, hi) - load.begin());
         load[s] += j.cost;
         b->slot_jobs[s].push_back(j);
     }
@@ -347,15 +378,15 @@ extern "C" pf_status pf_batch_create(pf_ctx *ctx, int32_t n, const pf_batch_inst
     b->nstreams = n_streams;
     pf_status s = batch_build(b, tol);
     if (s == PF_OK) {
-        b->streams.resize(n_streams);
-        for (int k = 0; k < n_streams && s == PF_OK; ++k)
-            if (cudaStreamCreateWithFlags(&b->streams[k], cudaStreamNonBlocking) != cudaSuccess)
+        b->streams.resize(b->nstreams);
+        for (auto &t : b->streams)
+            if (s == PF_OK && cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking) != cudaSuccess)
                 s = PF_ERR_CUDA;
         if (s == PF_OK &&
             (cudaStreamCreateWithFlags(&b->direct_stream, cudaStreamNonBlocking) != cudaSuccess ||
              cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking) != cudaSuccess))
             s = PF_ERR_CUDA;
-        b->events.resize(n_streams + 3);
+        b->events.resize(b->nstreams + 3);
         for (auto &e : b->events)
             if (s == PF_OK && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) != cudaSuccess)
                 s = PF_ERR_CUDA;
@@ -376,6 +407,7 @@ extern "C" pf_status pf_batch_create(pf_ctx *ctx, int32_t n, const pf_batch_inst
             }
         }
     }
+    batch_free_streams(b);
     if (s == PF_OK) {
         cudaError_t e = cudaGraphInstantiate(&b->exec, b->graph, 0);
         if (e != cudaSuccess) {

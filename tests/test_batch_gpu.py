@@ -126,3 +126,23 @@ def test_batch_of_256_simulations_equals_alone_and_oracle():
         assert normwise_err(res[i]["vx"].cpu().numpy()[idx], res[i]["vy"].cpu().numpy()[idx],
                             rx, ry) <= 1e-6, (i, methods[i])
     bt.close()
+
+
+@pytest.mark.parametrize("streams", [1, 2, 64])
+@pytest.mark.parametrize("remesh", [False, True])
+def test_remeshes_on_streams_of_their_own(streams, remesh):
+    """One stream (everything in series), fewer and more remesh streams than
+    sets, and no remesh at all: bitwise the single calls, twice."""
+    from pfblob.batch import Batch
+    sims = make_sims([2500, 40000, 900])
+    bt = Batch(sims, tol=1e-6, n_streams=streams, remesh=remesh)
+    for _ in range(2):
+        bt.run()
+        for s, r in zip(sims, bt.results()):
+            assert r["status"] == 0
+            vx, vy, xn, yn, gn = alone(s, r["method"], r["leaf_level"])
+            assert torch.equal(vx, r["vx"]) and torch.equal(vy, r["vy"])
+            if remesh:
+                assert torch.equal(xn, r["x"]) and torch.equal(yn, r["y"])
+                assert torch.equal(gn, r["g"])
+    bt.close()
