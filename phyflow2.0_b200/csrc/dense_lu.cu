@@ -456,8 +456,11 @@ k_lu_stripe(int64_t m, int j0, int nb, double *__restrict__ A, const int32_t *__
     }
 }
 
-// Back substitution of one block with a division per unknown, for diagonals
-// that do not allow scaling the rows first (out of line: rarely taken).
+// Back substitution of one block with a division per unknown, for blocks whose
+// rows can't be divided by their diagonals first.  v, d: right-hand side and
+// diagonal of the lane's row; t: the block's entries of U, negated.  (Out of line
+// and with the entries in shared memory: inlined, or reading U again, the rarely
+// taken path costs the usual one 6% by register allocation.)
 __device__ __noinline__ double back_unscaled(double v, double d, const double (*t)[33]) {
     const int lane = threadIdx.x & 31;
 #pragma unroll 1
@@ -472,9 +475,12 @@ __device__ __noinline__ double back_unscaled(double v, double d, const double (*
 // One substitution (BACK: with U from the last block up, else with the unit
 // lower L from the first down) of k_lu_solve, by blocks of 32 unknowns.
 //   s_t[buf]: the block's triangle, negated, zero elsewhere (BACK: each row
-//     divided by its diagonal, which keeps the division out of the chain; a
-//     block with a diagonal that is zero, not finite or near the ends of the
-//     range is left unscaled and divides unknown by unknown);
+//     divided by its diagonal, which keeps the division out of the chain);
+//   s_u[buf]: BACK: the triangle as it is.  The scaled one holds while every
+//     quotient of the block is a normal number.  A block with another one or with
+//     a diagonal that is zero or not finite (s_raw), and one whose scaled solution
+//     is not finite (its right-hand side may overflow when it is divided before
+//     the others' shares are taken off), is solved from s_u, unknown by unknown;
 //   thread (wid, rq, cq) of the CTA works on columns cq + 8 q of rows
 //     64 i + 4 wid + rq: the first LV_PRE row passes' factors are loaded
 //     while another warp solves the triangle, and their products with the
@@ -482,7 +488,7 @@ __device__ __noinline__ double back_unscaled(double v, double d, const double (*
 template <bool BACK>
 __device__ __forceinline__ void lu_substitute(int64_t m, const double *__restrict__ LU,
                                               double *b, double (*s_t)[32][33],
-                                              double (*s_d)[32], int *s_raw, double *s_x) {
+                                              double (*s_u)[32][33], double (*s_d)[32], int *s_raw, double *s_x) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     static_assert(LV_ROW_WARPS == 16, "two rows of a triangle per warp, 64 rows per pass");
     const bool solver = wid == LV_ROW_WARPS;  // the triangles' warp
@@ -506,11 +512,11 @@ __device__ __forceinline__ void lu_substitute(int64_t m, const double *__restric
             if (BACK) {
                 // (zeros divide d by itself: a zero would take the division's slow path)
                 const double sc = (v != 0.0 ? v : dg[h]) / dg[h];
-                const bool ok = fabs(dg[h]) > 1e-100 && fabs(dg[h]) < 1e100 && fabs(sc) < 1e100;
-                if (__all_sync(0xffffffffu, ok))
-                    v = v != 0.0 ? sc : 0.0;
-                else if (lane == 0)
-                    s_raw[buf] |= 1;  // any writer: the same value
+                const unsigned ex = __double2hiint(sc) >> 20 & 0x7ff;
+                const bool ok = ex - 1u < 0x7feu;  // a normal number
+                if (!__all_sync(0xffffffffu, ok) && lane == 0) s_raw[buf] = 1;  // any writer: the same
+                s_u[buf][w][lane] = v;
+                v = v != 0.0 ? sc : 0.0;
                 __syncwarp();
                 if (lane == 0) s_d[buf][w] = dg[h];
             }
@@ -554,13 +560,16 @@ __device__ __forceinline__ void lu_substitute(int64_t m, const double *__restric
         if (solver) {
             const bool in = j0 + lane < m;
             double v = in ? b[j0 + lane] : 0.0;
-            if (BACK && s_raw[buf]) {
-                v = back_unscaled(v, s_d[buf][lane], s_t[buf]);
-            } else if (BACK) {
-                v = v / s_d[buf][lane];
+            if (BACK) {
+                bool raw = s_raw[buf] != 0;
+                if (!raw) {
+                    v = v / s_d[buf][lane];
 #pragma unroll
-                for (int k = 31; k > 0; --k)
-                    v = fma(s_t[buf][lane][k], __shfl_sync(0xffffffffu, v, k), v);
+                    for (int k = 31; k > 0; --k)
+                        v = fma(s_t[buf][lane][k], __shfl_sync(0xffffffffu, v, k), v);
+                    raw = __any_sync(0xffffffffu, (__double2hiint(v) >> 20 & 0x7ff) == 0x7ff);
+                }
+                if (raw) v = back_unscaled(in ? b[j0 + lane] : 0.0, s_d[buf][lane], s_u[buf]);
             } else {
 #pragma unroll
                 for (int k = 0; k < 31; ++k)
@@ -621,7 +630,7 @@ __global__ void __launch_bounds__(LV_THREADS)
 k_lu_solve(int64_t m, const double *__restrict__ LU, const int32_t *__restrict__ ipiv,
            double *bg) {
     extern __shared__ __align__(16) double s_b[];
-    __shared__ double s_t[2][32][33];
+    __shared__ double s_t[2][32][33], s_u[2][32][33];
     __shared__ double s_d[2][32], s_x[32];
     __shared__ int s_raw[2];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -651,8 +660,8 @@ k_lu_solve(int64_t m, const double *__restrict__ LU, const int32_t *__restrict__
         }
         __syncthreads();
     }
-    lu_substitute<false>(m, LU, b, s_t, s_d, s_raw, s_x);
-    lu_substitute<true>(m, LU, b, s_t, s_d, s_raw, s_x);
+    lu_substitute<false>(m, LU, b, s_t, s_u, s_d, s_raw, s_x);
+    lu_substitute<true>(m, LU, b, s_t, s_u, s_d, s_raw, s_x);
     if (SM)
         for (int64_t i = threadIdx.x; i < m; i += LV_THREADS) bg[i] = s_b[i];
 }
