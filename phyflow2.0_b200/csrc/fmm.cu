@@ -1614,7 +1614,9 @@ pf_status velocity_fmm(pf_ctx *ctx, int64_t n_src, const double *x, const double
         const int cap = ctx->num_sms * 4;  // each CTA ends in an atomic on the ticket
         PF_TRY(pf::arena_reserve(ctx, pf::align256(cap * sizeof(BBox))));
         BBox *part = static_cast<BBox *>(pf::arena_take(ctx, cap * sizeof(BBox)));
-        const int64_t nt_box = (xt == x && yt == y) ? 0 : n_tgt;
+        // targets that are the sources, or the first of them, are in their box (sources
+        // that are the first of the targets, the same pointers, don't cover them)
+        const int64_t nt_box = (xt == x && yt == y && n_tgt <= n_src) ? 0 : n_tgt;
         const int64_t nb = std::min<int64_t>(pf::ceil_div(n_src + nt_box, 256), cap);
         k_bbox<<<(unsigned)nb, 256, 0, st>>>(
             x, y, n_src, xt, yt, nt_box, part,

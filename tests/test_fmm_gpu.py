@@ -366,3 +366,27 @@ def test_tree_of_every_leaf_level(leaf_level, n, nt):
     assert np.array_equal(out[0][0], out[1][0]) and np.array_equal(out[0][1], out[1][1])
     rx, ry = oracle.velocity_direct(x, y, g, 2 * sigma * sigma, xt, yt)
     assert normwise_err(*out[0], rx, ry) <= TOL
+
+
+@pytest.mark.parametrize("n_src,n_tgt", [(5000, 12000), (4096, 4097), (9000, 3000)])
+def test_sources_and_targets_of_one_array(n_src, n_tgt):
+    """Sources and targets that begin at the same address: the targets behind the
+    last source lie outside the sources' box and count for the tree's box and
+    for the check of the coordinates."""
+    import pfblob
+    rng = np.random.default_rng(n_src)
+    n = max(n_src, n_tgt)
+    x, y = rng.random(n), rng.random(n)
+    x[n_src:] = rng.uniform(-2.0, 3.0, n - n_src)
+    y[n_src:] = rng.uniform(-2.0, 3.0, n - n_src)
+    g = rng.standard_normal(n_src) / n_src
+    X, Y, G = T(x), T(y), T(g)
+    v = pfblob.velocity(X[:n_src], Y[:n_src], G, 0.01, method=pfblob.FMM_METHOD,
+                        xEval=X[:n_tgt], yEval=Y[:n_tgt])
+    rx, ry = oracle.velocity_direct(x[:n_src], y[:n_src], g, 2e-4, x[:n_tgt], y[:n_tgt])
+    assert normwise_err(v[0].cpu().numpy(), v[1].cpu().numpy(), rx, ry) <= TOL
+    if n_tgt > n_src:
+        X[n_tgt - 1] = float("nan")
+        with pytest.raises(Exception, match="NaN"):
+            pfblob.velocity(X[:n_src], Y[:n_src], G, 0.01, method=pfblob.FMM_METHOD,
+                            xEval=X[:n_tgt], yEval=Y[:n_tgt])
