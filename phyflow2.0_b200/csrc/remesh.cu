@@ -47,6 +47,7 @@
 #include <vector>
 
 #include "remesh.cuh"
+#include "scan.cuh"
 #include "segsort.cuh"
 
 namespace {
@@ -1040,10 +1041,15 @@ cudaError_t tile_smem_attr() {
 // kept cells of each part of KP_TILE cells; k_rm_keep_emit adds the earlier
 // parts' counts itself, ranks its cells by ballots and writes the new blobs.
 // (Flags, a three-pass scan of slots and the emission as five launches took 25
-// us for 711,000 cells; these take 14.)
+// us for 711,000 cells; these take 14.)  Every CTA reading every count is
+// quadratic in the parts, so beyond KP_SELF of them (16 loads a thread, 8 million
+// cells) the counts are scanned first.  The scan costs 3.5 us, the reading 2 us at
+// 4096 parts, 120 at 64 million cells and 24.5 ms at 729 million (12 million
+// blobs: a call 76.2 ms, scanned 51.7).
 constexpr int KP_THREADS = 256;
 constexpr int KP_STEPS = 8;  // 32 cells per warp and step
 constexpr int KP_TILE = KP_THREADS * KP_STEPS;
+constexpr int64_t KP_SELF = 16 * KP_THREADS;
 
 __device__ __forceinline__ unsigned keep_ballot(const Win &w, int64_t cid,
                                                 const int32_t *__restrict__ flag,
@@ -1064,9 +1070,12 @@ k_rm_keep_count(const RmHead *__restrict__ hd, const int32_t *__restrict__ flag,
                 int32_t *__restrict__ tsum) {
     __shared__ int s_w[KP_THREADS / 32];
     Win w;
-    if (!load_win(hd, w)) return;
+    const bool ok = load_win(hd, w);
     const int64_t t0 = (int64_t)blockIdx.x * KP_TILE;
-    if (t0 >= w.ncell) return;
+    if (!ok || t0 >= w.ncell) {
+        if (threadIdx.x == 0) tsum[blockIdx.x] = 0;
+        return;
+    }
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const double thr = pc->thr;
     int n = 0;
@@ -1082,10 +1091,11 @@ k_rm_keep_count(const RmHead *__restrict__ hd, const int32_t *__restrict__ flag,
     }
 }
 
+// scanned: tsum holds the counts' exclusive sums, hd->total their sum
 __global__ void __launch_bounds__(KP_THREADS)
 k_rm_keep_emit(RmHead *__restrict__ hd, WParams wp, const int32_t *__restrict__ flag,
                const double *__restrict__ acc, const pf::PcState *__restrict__ pc,
-               const int32_t *__restrict__ tsum, int64_t capacity, double *__restrict__ xo,
+               const int32_t *__restrict__ tsum, bool scanned, int64_t capacity, double *__restrict__ xo,
                double *__restrict__ yo, double *__restrict__ go, int64_t *__restrict__ ixo,
                int64_t *__restrict__ iyo) {
     __shared__ int s_w[KP_THREADS / 32], s_pre[KP_THREADS / 32], s_tot[KP_THREADS / 32];
@@ -1095,8 +1105,12 @@ k_rm_keep_emit(RmHead *__restrict__ hd, WParams wp, const int32_t *__restrict__ 
     if (t0 >= w.ncell) return;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const double thr = pc->thr;
-    const int ntiles = (int)((w.ncell + KP_TILE - 1) / KP_TILE);
+    const int ntiles = scanned ? 0 : (int)((w.ncell + KP_TILE - 1) / KP_TILE);
     int pre = 0, tot = 0;  // kept cells of the earlier parts, and of all
+    if (scanned && threadIdx.x == 0) {
+        pre = tsum[blockIdx.x];
+        tot = hd->total;
+    }
     for (int j = threadIdx.x; j < ntiles; j += KP_THREADS) {
         const int c = tsum[j];
         tot += c;
@@ -1124,7 +1138,7 @@ k_rm_keep_emit(RmHead *__restrict__ hd, WParams wp, const int32_t *__restrict__ 
         at += s_pre[k] + (k < wid ? s_w[k] : 0);
         all += s_tot[k];
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) hd->total = (int32_t)all;
+    if (!scanned && blockIdx.x == 0 && threadIdx.x == 0) hd->total = (int32_t)all;
     if (all > capacity) return;  // capacity error: write nothing
 #pragma unroll
     for (int k = 0; k < KP_STEPS; ++k) {
@@ -1308,12 +1322,14 @@ pf_status remesh_core(Bump &sc, int64_t n, const double *x, const double *y, con
     }
     if (cells) {
         PF_TRY(popctl_decide(sc, cap_cell, acc, flag, *pc, st, &hd->ncell));
-        // the slots' array is free in this mode: the parts' counts
-        const unsigned gk = (unsigned)ceil_div(cap_cell, KP_TILE);
-        k_rm_keep_count<<<gk, KP_THREADS, 0, st>>>(hd, flag, acc, pc->state, slot);
+        // the slots' array is free in this mode: the parts' counts (and the scan's scratch)
+        const int64_t gk = ceil_div(cap_cell, KP_TILE);
+        const bool scanned = gk > KP_SELF;
+        k_rm_keep_count<<<(unsigned)gk, KP_THREADS, 0, st>>>(hd, flag, acc, pc->state, slot);
         PF_TRY(launch_status("k_rm_keep_count"));
-        k_rm_keep_emit<<<gk, KP_THREADS, 0, st>>>(hd, wp, flag, acc, pc->state, slot, capacity, xo, yo,
-                                                  go, ixo, iyo);
+        if (scanned) PF_TRY(exclusive_scan_i32(slot, slot, gk, slot + gk, &hd->total, st));
+        k_rm_keep_emit<<<(unsigned)gk, KP_THREADS, 0, st>>>(hd, wp, flag, acc, pc->state, slot, scanned,
+                                                            capacity, xo, yo, go, ixo, iyo);
         PF_TRY(launch_status("k_rm_keep_emit"));
     }
     if (!total && !bad) return PF_OK;

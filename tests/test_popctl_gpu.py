@@ -124,3 +124,23 @@ def test_fused_control_at_part_edges(nx, ny):
     rx, ry, rg = pfblob.remesh_device(*t, h, -1.5 * h, -1.5 * h)
     px, py, pg, pt = pfblob.population_control_device(rx, ry, rg, *thr)
     assert torch.equal(fx, px) and torch.equal(fy, py) and torch.equal(fg, pg) and ft == pt
+
+
+@pytest.mark.parametrize("side", [2893, 2897, 4001])
+def test_fused_control_in_a_wide_window(side):
+    """Few blobs in a window of about 8 million cells and more, from where the
+    parts' counts are scanned in launches of their own: exactly the remesh followed by
+    PopulationControl."""
+    import pfblob
+    rng = np.random.default_rng(side)
+    n, h = 200_000, 1.0 / 1024
+    x, y = rng.random(n) * (side * h), rng.random(n) * (side * h)
+    x[:2], y[:2] = (0.0, side * h), (0.0, side * h)
+    g = np.where(rng.random(n) < 0.3, 1.0, 1e-14) * rng.standard_normal(n)
+    t = [torch.from_numpy(a).cuda() for a in (x, y, g)]
+    thr = (1e-8, 1e-8)
+    for _ in range(2):  # the second call's scratch is sized by the first one's window
+        fx, fy, fg, ft = pfblob.remesh_device(*t, h, -1.5 * h, -1.5 * h, population_control=thr)
+        rx, ry, rg = pfblob.remesh_device(*t, h, -1.5 * h, -1.5 * h)
+        px, py, pg, pt = pfblob.population_control_device(rx, ry, rg, *thr)
+        assert torch.equal(fx, px) and torch.equal(fy, py) and torch.equal(fg, pg) and ft == pt
