@@ -798,25 +798,48 @@ k_p2p_runs(int L, int kb, const int2 *__restrict__ q, int nq, int nqp,
     if (!runs && threadIdx.x == 0) nruns_or_off[b] = s_n;
 }
 
-// The target groups beyond a block's first, as (block, group): their CTAs run
-// beside the first groups' instead of after them in one CTA (1.8e6 blobs in an
-// annulus, three groups in each occupied block: P2P 2.34 -> 2.02 ms).  Each
-// group is computed by one CTA, so results do not depend on the list's order.
-__device__ __forceinline__ void list_more_groups(const P2PDesc &d, int64_t i) {
-    if (i >= d.nblk) return;
-    const int b = d.order[i];
-    int t0;
-    const int ngrp = p2p_groups(p2p_targets(d, b, t0));
-    if (ngrp < 2) return;
-    const int64_t at = atomicAdd(d.nmore, (unsigned)(ngrp - 1));
-    for (int g = 1; g < ngrp; ++g)
-        if (PF_IDX_OK(at + g - 1, d.more_cap, 207)) d.more[at + g - 1] = make_int2(b, g);
+// Lists the target groups that are not tasks by themselves, as (block, group), of
+// 256 blocks of the launch order per CTA: those beyond a block's first, whose
+// CTAs run beside the first groups' instead of after them in one CTA (1.8e6 blobs
+// in an annulus, three groups in each occupied block: P2P 2.34 -> 2.02 ms), or
+// all, see P2P_DIRECT_MAX.  Each group is computed by one CTA, so results do not
+// depend on the list's order; a block's groups are next to each other in it.
+__device__ __forceinline__ void list_groups(const P2PDesc &d, int64_t i) {
+    __shared__ int s_sum[8];
+    __shared__ unsigned s_at;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int g0 = d.direct ? 1 : 0;
+    int b = 0, ngrp = 0;
+    if (i < d.nblk) {
+        b = d.order[i];
+        int t0;
+        ngrp = p2p_groups(p2p_targets(d, b, t0));
+    }
+    const int n = max(ngrp - g0, 0);
+    int inc = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int t = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += t;
+    }
+    if (lane == 31) s_sum[wid] = inc;
+    __syncthreads();
+    int pre = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) {
+        if (w < wid) pre += s_sum[w];
+        all += s_sum[w];
+    }
+    if (threadIdx.x == 0 && all) s_at = atomicAdd(d.nmore, (unsigned)all);
+    __syncthreads();
+    const int64_t at = (int64_t)s_at + pre + inc - n;
+    for (int k = 0; k < n; ++k)
+        if (PF_IDX_OK(at + k, d.more_cap, 207)) d.more[at + k] = make_int2(b, g0 + k);
 }
 
 // Second half of the counting sort, and what else needs only the leaf counts
 // and starts, in CTAs after the sort's gn: nc CTAs sum the counts up `nlev`
-// levels from the leaves (L), the rest list the P2P groups beyond each block's
-// first (d.nblk = 0: none).  As launches of their own the two cost 2-4 us each
+// levels from the leaves (L), the rest list P2P groups (d.nblk = 0: none).  As launches of their own the two cost 2-4 us each
 // with their gaps.
 __global__ void __launch_bounds__(256)
 k_place(int64_t n, const uint32_t *__restrict__ key, const int32_t *__restrict__ rank,
@@ -824,7 +847,7 @@ k_place(int64_t n, const uint32_t *__restrict__ key, const int32_t *__restrict__
         int32_t *__restrict__ big_n, unsigned gn, int L, int nlev, unsigned nc, int32_t *cnt_all,
         const P2PDesc d) {
     if (blockIdx.x >= gn + nc) {
-        list_more_groups(d, (int64_t)(blockIdx.x - gn - nc) * 256 + threadIdx.x);
+        list_groups(d, (int64_t)(blockIdx.x - gn - nc) * 256 + threadIdx.x);
         return;
     }
     if (blockIdx.x >= gn) {
@@ -840,21 +863,21 @@ k_place(int64_t n, const uint32_t *__restrict__ key, const int32_t *__restrict__
     if (rank[i] == LEAF_SMALL) big[atomicAdd(big_n, 1)] = (int32_t)key[i];
 }
 
-// One CTA (one warp) per target group: CTA i < nblk the first group of block i
-// of the launch order (heaviest first), the CTAs after those the other groups
+// One CTA (one warp) per target group: CTA i < direct the first group of block i
+// of the launch order (heaviest first), the CTAs after those the listed groups
 // (several each where clusters make more of them than CTAs).
 __global__ void __launch_bounds__(32, P2P_MIN_CTAS) k_p2p(const P2PDesc d) {
     __shared__ P2PSmem sm;
-    const unsigned nblk = (unsigned)d.nblk;
+    const unsigned direct = (unsigned)d.direct;
 #pragma unroll 1
-    for (unsigned t = blockIdx.x;; t += gridDim.x - nblk) {
+    for (unsigned t = blockIdx.x;; t += gridDim.x - direct) {
         int b, gi;
         if (!p2p_task(d, t, b, gi)) return;
         int t0;
         const int tn = p2p_targets(d, b, t0);
         if (tn == 0) return;
         p2p_group(d, b, t0, tn, gi, sm);
-        if (t < nblk) return;
+        if (t < direct) return;
     }
 }
 
@@ -1174,11 +1197,28 @@ static int p2p_warps(int64_t nblk, int64_t nt, int64_t nt_beside) {
     return groups <= 600 ? 8 : groups <= 2200 ? 4 : 1;
 }
 
-// CTAs for the groups beyond the blocks' first: those of a layer around a body,
-// or what the device holds (mostly idle CTAs for every group there could be
-// cost 13 us at 2^20 uniform blobs).
-static int64_t p2p_more_ctas(int64_t nblk, int64_t nt, int64_t more_cap) {
-    return std::min<int64_t>(more_cap, std::max<int64_t>(148 * P2P_MIN_CTAS, nt / 60 - nblk));
+// Blocks up to which each block's first group is a CTA by itself, the heaviest
+// blocks first; beyond, all groups are listed.  Uniform sets of 2^18 to 2^20 blobs
+// lose 2-4% of P2P when listed, by the order of the last CTAs.  From 65,536 blocks
+// on that is 0.3%, and the empty blocks' CTAs and the second groups being far
+// from the first cost more: 2^22 blobs in an annulus, P2P 3.10 ms, listed 2.77 (one
+// CTA per block for all its groups 2.97).
+constexpr int64_t P2P_DIRECT_MAX = 32768;
+
+static int64_t p2p_direct(int64_t nblk) { return nblk <= P2P_DIRECT_MAX ? nblk : 0; }
+
+// Most groups that can be listed.
+static int64_t p2p_more_cap(int64_t nblk, int64_t nt) {
+    return nt / P2P_GROUP + 1 + nblk - p2p_direct(nblk);
+}
+
+// CTAs for the listed groups: those of a layer around a body, or what the device
+// holds (mostly idle CTAs for every group there could be cost 13 us at 2^20
+// uniform blobs).
+static int64_t p2p_more_ctas(int64_t nblk, int64_t nt) {
+    const int64_t direct = p2p_direct(nblk);
+    return std::min<int64_t>(p2p_more_cap(nblk, nt),
+                             std::max<int64_t>({148 * P2P_MIN_CTAS, nblk - direct, nt / 60 - direct}));
 }
 
 static size_t fmm_scratch_bytes(const FmmCache &c, int64_t ns, int64_t nt, bool same) {
@@ -1200,7 +1240,7 @@ static size_t fmm_scratch_bytes(const FmmCache &c, int64_t ns, int64_t nt, bool 
     add(16 * (size_t)nbox * NP); add(16 * (size_t)nbox * NP);  // M, L
     add(16 * nt);                                   // near velocities
     add(4 * (std::max(ns, nt) / (LEAF_SMALL + 1) + 3));  // leaves for the segment sort
-    add(8 * (size_t)(nt / P2P_GROUP + 1));          // P2P groups beyond the first
+    add(8 * (size_t)p2p_more_cap((int64_t)1 << (2 * (L - c.kb)), nt));  // P2P groups listed
     add(4 * pf::scan_tmp_ints(nleaf));
     return need + 4096;
 }
@@ -1250,8 +1290,9 @@ static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, dou
     double2 *nearv = (double2 *)take(16 * nt);
     // leaves listed for the segment sort: [0] count, [1 ..] leaf ids
     int32_t *big = (int32_t *)take(4 * (std::max(ns, nt) / (LEAF_SMALL + 1) + 3));
-    // P2P groups beyond each block's first
-    const int64_t more_cap = nt / P2P_GROUP + 1;
+    // P2P groups that are listed
+    const int64_t nblk = (int64_t)1 << (2 * (L - kb));
+    const int64_t more_cap = p2p_more_cap(nblk, nt);
     int2 *more = (int2 *)take(8 * (size_t)more_cap);
     int32_t *tmp = (int32_t *)take(4 * pf::scan_tmp_ints(nleaf));
     if (!tmp) {
@@ -1268,9 +1309,9 @@ static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, dou
     }
 
     // the near field's description
-    const int64_t nblk = (int64_t)1 << (2 * (L - kb));
     P2PDesc pd;
     pd.nblk = nblk;
+    pd.direct = p2p_direct(nblk);
     pd.kb = kb;
     pd.tstart = tstart;
     pd.tcnt = T.cnt;
@@ -1311,9 +1352,9 @@ static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, dou
     const int warps = p2p_warps(nblk, nt, a.nt_beside);
     auto near = [&]() -> pf_status {
         if (warps > 1) {
-            PF_TRY(pf::fmmx::launch_p2p_multi(pd, warps, (unsigned)(nblk + more_cap), st));
+            PF_TRY(pf::fmmx::launch_p2p_multi(pd, warps, (unsigned)(pd.direct + more_cap), st));
         } else {
-            k_p2p<<<(unsigned)(nblk + p2p_more_ctas(nblk, nt, more_cap)), 32, 0, st>>>(pd);
+            k_p2p<<<(unsigned)(pd.direct + p2p_more_ctas(nblk, nt)), 32, 0, st>>>(pd);
             PF_TRY(pf::launch_status("k_p2p"));
         }
         return PF_OK;

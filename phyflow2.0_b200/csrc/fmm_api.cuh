@@ -52,9 +52,10 @@ struct P2PDesc {
     pfd::GaussParams gp;
     double2 *nearv;
     unsigned long long *pairs;
+    int64_t direct;      // blocks whose first groups are tasks by themselves: all or none
     unsigned *nmore;     // entries of more (a counter of the call, zeroed with the others)
-    int2 *more;          // (block, group) of the target groups beyond a block's first [more_cap]
-    int64_t more_cap;    // nt / 96 + 1 bounds them
+    int2 *more;          // (block, group) of the other target groups [more_cap]
+    int64_t more_cap;    // nt / 96 + 1 bounds them, and nblk more where none is direct
     int64_t ns, nt;      // sorted sources and targets (bounds-checked build)
 };
 

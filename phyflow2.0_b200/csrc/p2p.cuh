@@ -567,17 +567,17 @@ __device__ __forceinline__ int p2p_targets(const P2PDesc &d, int64_t b, int &t0)
 // Target groups of a block of tn targets.
 __device__ __forceinline__ int p2p_groups(int tn) { return (tn + P2P_GROUP - 1) / P2P_GROUP; }
 
-// Block and group of task t: t < nblk the first group of block t of the launch
+// Block and group of task t: t < direct the first group of block t of the launch
 // order, then the listed groups; false past those.
 __device__ __forceinline__ bool p2p_task(const P2PDesc &d, unsigned t, int &b, int &gi) {
-    const unsigned nblk = (unsigned)d.nblk;
-    if (t < nblk) {
+    const unsigned direct = (unsigned)d.direct;
+    if (t < direct) {
         b = d.order[t];
         gi = 0;
         return true;
     }
-    if (t - nblk >= *d.nmore) return false;
-    const int2 e = d.more[t - nblk];
+    if (t - direct >= *d.nmore) return false;
+    const int2 e = d.more[t - direct];
     b = e.x;
     gi = e.y;
     return true;

@@ -390,3 +390,35 @@ def test_sources_and_targets_of_one_array(n_src, n_tgt):
         with pytest.raises(Exception, match="NaN"):
             pfblob.velocity(X[:n_src], Y[:n_src], G, 0.01, method=pfblob.FMM_METHOD,
                             xEval=X[:n_tgt], yEval=Y[:n_tgt])
+
+
+@pytest.mark.parametrize("leaf_level", [8, 9, 10])
+@pytest.mark.parametrize("n", [9000, 130000])
+def test_near_field_group_lists(leaf_level, n):
+    """A layer around a body and a cluster, so that most blocks are empty and some
+    hold several target groups: up to 32,768 blocks (level 8) the first groups are
+    tasks by themselves, beyond all groups are listed, with several warps per
+    group (9,000) and with one; against the oracle, for the blobs and for
+    separate targets."""
+    from pfblob import _lib
+    from pfblob import workloads as wl
+    b = wl.shear_layer(n=n)
+    rng = np.random.default_rng(n + leaf_level)
+    x, y, g, sigma = b.x.copy(), b.y.copy(), b.g, 1e-3  # a core that level 10 can hold
+    k = n // 8
+    x[:k] = 1.2 + 1e-3 * rng.standard_normal(k)
+    y[:k] = 0.1 + 1e-3 * rng.standard_normal(k)
+    m = n // 2 + 1
+    xt, yt = np.append(rng.uniform(-1.5, 1.5, m - 500), x[:500]), \
+        np.append(rng.uniform(-1.5, 1.5, m - 500), y[:500] + 1e-4)
+    _lib.fmm_set_tuning(leaf_level, 0, 1)
+    try:
+        own = fmm(x, y, g, sigma)
+        assert _lib.fmm_last_stats(DEV.index)["leaf_level"] == leaf_level
+        far = fmm(x, y, g, sigma, xt, yt)
+    finally:
+        _lib.fmm_set_tuning(0, 0, 1)
+    for (vx, vy), (px, py) in ((own, (x, y)), (far, (xt, yt))):
+        sub = np.append(rng.choice(px.size, 1200, replace=False), np.arange(200))
+        rx, ry = oracle.velocity_direct(x, y, g, 2 * sigma * sigma, px[sub].copy(), py[sub].copy())
+        assert normwise_err(vx[sub], vy[sub], rx, ry) <= TOL
