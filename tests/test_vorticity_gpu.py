@@ -86,3 +86,44 @@ def test_sources_beyond_reach_add_nothing(n, order):
         gb[x.size // 3] = bad
         assert np.isnan(pfblob.vorticity(x, y, gb, sigma, xEval=np.array([900.0]),
                                          yEval=np.array([-900.0]))).all()
+
+
+@pytest.mark.parametrize("ns,nt,order", [(9216, 9216, "lattice"), (9409, 9409, "lattice"),
+                                         (12100, 12100, "lattice"), (18225, 18225, "lattice"),
+                                         (9500, 9500, "random"), (13000, 13001, "clusters"),
+                                         (150001, 700, "random"), (33, 3000001, "lattice")])
+def test_tested_and_untested_sets(ns, nt, order):
+    """Around the number of pairs from which sources are tested (8.5e7), one wave of
+    CTAs and several, many sources for few targets and the reverse: against the
+    FP64 oracle, 1e-6 as above; the strengths of sources beyond every target's
+    reach change no bit; a source that is not finite still reaches all."""
+    import pfblob
+    rng = np.random.default_rng(ns + nt)
+
+    def points(n):
+        if order == "lattice":
+            s = int(np.ceil(np.sqrt(n)))
+            c = -1.0 + (np.arange(s) + 0.5) * (2.0 / s)
+            return [a.ravel()[:n].copy() for a in np.meshgrid(c, c, indexing="ij")]
+        x, y = rng.uniform(-1, 1, n), rng.uniform(-1, 1, n)
+        if order == "clusters":
+            x[n // 2:] += 50.0
+        return [x, y]
+
+    x, y = points(ns)
+    xt, yt = (x, y) if nt == ns else points(nt)
+    g = rng.standard_normal(ns) / ns
+    sigma = 2.5 / np.sqrt(max(ns, nt))
+    far = rng.choice(ns, ns // 10, replace=False)
+    y[far] = 200.0
+    if nt == ns:
+        yt = np.where(np.isin(np.arange(ns), far), 0.5, y)
+    w = pfblob.vorticity(x, y, g, sigma, xEval=xt, yEval=yt)
+    sub = rng.choice(nt, min(nt, 2000), replace=False)
+    r = oracle.vorticity_direct(x, y, g, 2 * sigma * sigma, xt[sub].copy(), yt[sub].copy())
+    assert err(w[sub], r) <= TOL
+    g2 = g.copy()
+    g2[far] *= 1e6
+    assert np.array_equal(w, pfblob.vorticity(x, y, g2, sigma, xEval=xt, yEval=yt))
+    g2[far[0]] = np.inf
+    assert np.isnan(pfblob.vorticity(x, y, g2, sigma, xEval=xt, yEval=yt)).all()
