@@ -303,10 +303,10 @@ static pf_status batch_enqueue(pf_batch *b) {
     // the persistent direct kernel
     PF_TRY(pf::launch_direct_batch(b->d_dinst, b->d_items, b->n_items, b->d_red_items, b->n_red,
                                    b->d_counter, b->direct_grid, b->direct_stream));
-    int64_t nt_all = 0;  // targets of all FMM sets: they share the device
+    int64_t groups = 0;  // P2P groups of all FMM sets: they share the device
     for (int s = 0; s < S; ++s)
         for (const Job &j : b->slot_jobs[s])
-            if (j.kind == 0) nt_all += b->inst[j.inst].n;
+            if (j.kind == 0) groups += pf::fmmx::plan_groups(b->plans[j.inst], b->inst[j.inst].n);
     for (int s = 0; s < S; ++s) {
         cudaStream_t st = b->streams[s];
         for (const Job &j : b->slot_jobs[s]) {
@@ -314,7 +314,8 @@ static pf_status batch_enqueue(pf_batch *b) {
             pf::Bump sc{b->slot_scratch[s], b->slot_bytes[s], 0};
             if (j.kind == 0) {
                 PF_TRY(pf::fmmx::plan_exec(b->plans[j.inst], sc, d.n, d.x, d.y, d.g, d.n, d.x, d.y,
-                                           d.ksigmasqr, d.vx, d.vy, nt_all - d.n,
+                                           d.ksigmasqr, d.vx, d.vy,
+                                           groups - pf::fmmx::plan_groups(b->plans[j.inst], d.n),
                                            b->d_ctr + pf::fmmx::FMM_COUNTERS * s, nullptr, st));
             } else {
                 const int64_t nbx = b->nbx[j.inst], nby = b->nby[j.inst];

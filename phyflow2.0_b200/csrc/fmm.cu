@@ -1182,18 +1182,27 @@ struct FmmArgs {
     double ksigmasqr, cutoff, tol;
     int ndirect;
     double *vx, *vy;
-    int64_t nt_beside = 0;  // targets of other sets whose calls run beside this one
+    int64_t groups_beside = 0;  // P2P groups of other sets whose calls run beside this one
 };
 
+// P2P target groups to expect: one per block and one more per 96 targets, but no
+// more than the blocks of a partly filled tree can hold, 40 targets each or, in
+// a tree of finer leaves, half as many again as a block has on average.
+static int64_t p2p_groups_expected(int64_t nblk, int64_t nt) {
+    const int64_t each = std::min<int64_t>(40, std::max<int64_t>(8, 3 * nt / (2 * nblk)));
+    return std::min<int64_t>(nblk + nt / P2P_GROUP, nt / each);
+}
+
 // Warps per target group (the result is the same), from the number of groups to
-// expect, this set's and those of the sets beside it in a batch: the device
-// holds 2960 one-warp CTAs (20 per SM), and one group alone is a serial chain of
-// 40-100 chunks; several warps cost barriers and exchanges, 40-75% where the
-// device is full.  P2P time with 1 / 4 / 8 warps, uniform sets: 3,001 blobs 73 /
+// expect, this set's and (two thirds of) those of the sets beside it in a batch:
+// the device holds 20 one-warp CTAs per SM, and one group alone is a serial
+// chain of 40-100 chunks; several warps cost barriers and exchanges, 40-75% where
+// the device is full.  P2P time with 1 / 4 / 8 warps, uniform sets: 3,001 blobs 73 /
 // 42 / 30 us; 30,000 163 / 89 / 79; 38,000 87 / 81 / 93; 100,000 185 / 163 / 187;
-// 140,000 230 / 234 / 273; 150,000 198 / 280 / 325.
-static int p2p_warps(int64_t nblk, int64_t nt, int64_t nt_beside) {
-    const int64_t groups = std::min<int64_t>(nblk + nt / P2P_GROUP, nt / 40) + nt_beside / 60;
+// 140,000 230 / 234 / 273; 150,000 198 / 280 / 325.  A call in a tree of finer
+// leaves, 62,384 blobs at level 7: 280 / 333 / 408, 15,129 at level 6: 125 / 132 / 152.
+static int p2p_warps(int64_t nblk, int64_t nt, int64_t groups_beside) {
+    const int64_t groups = p2p_groups_expected(nblk, nt) + 2 * groups_beside / 3;
     return groups <= 600 ? 8 : groups <= 2200 ? 4 : 1;
 }
 
@@ -1349,7 +1358,7 @@ static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, dou
     if (same) T = S;  // sort_points replaced S.perm by the final permutation
 
     PF_TRY(mark(1));
-    const int warps = p2p_warps(nblk, nt, a.nt_beside);
+    const int warps = p2p_warps(nblk, nt, a.groups_beside);
     auto near = [&]() -> pf_status {
         if (warps > 1) {
             PF_TRY(pf::fmmx::launch_p2p_multi(pd, warps, (unsigned)(pd.direct + more_cap), st));
@@ -1385,7 +1394,7 @@ static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, dou
         const int B = 1 << kb, Bp = B > 2 ? B : 2;
         {
             const int64_t nquad = (nbox - level_off(2)) / 4;  // box quads of levels 2..L
-            if (nquad <= M2L_AHEAD_QUADS && a.nt_beside == 0)
+            if (nquad <= M2L_AHEAD_QUADS && a.groups_beside == 0)
                 k_m2l<NP, true><<<(unsigned)nquad, 32, 0, fs>>>(
                     L, Bp, nquad, scnt_all, tcnt_all, M, Lc, c.d_far, c.d_far_ptr, c.maxpos, c.d_pw,
                     c.d_bin, ctr + 1);
@@ -1804,11 +1813,15 @@ size_t plan_scratch(const Plan *p, int64_t ns, int64_t nt, bool same) {
     return fmm_scratch_bytes(p->c, ns, nt, same);
 }
 
+int64_t plan_groups(const Plan *p, int64_t nt) {
+    return p2p_groups_expected((int64_t)1 << (2 * (p->c.L - p->c.kb)), nt);
+}
+
 pf_status plan_exec(const Plan *p, Bump &sc, int64_t ns, const double *x, const double *y,
                     const double *g, int64_t nt, const double *xt, const double *yt,
-                    double ksigmasqr, double *vx, double *vy, int64_t nt_beside,
+                    double ksigmasqr, double *vx, double *vy, int64_t groups_beside,
                     unsigned long long *ctr, cudaEvent_t *ev, cudaStream_t st) {
-    FmmArgs a{ns, nt, x, y, g, xt, yt, ksigmasqr, 0.0, 0.0, 0, vx, vy, nt_beside};
+    FmmArgs a{ns, nt, x, y, g, xt, yt, ksigmasqr, 0.0, 0.0, 0, vx, vy, groups_beside};
     return fmm_exec(p->c, p->x0, p->y0, p->w0, sc, a, ctr, ev, nullptr, st);
 }
 

@@ -20,9 +20,12 @@ pf_status plan_build(Plan *p, int L, int kb, int np, double x0, double y0, doubl
                      double cutoff, bool *p2p_ok);
 int plan_level(const Plan *p);
 size_t plan_scratch(const Plan *p, int64_t ns, int64_t nt, bool same);
+// P2P target groups to expect of nt targets
+int64_t plan_groups(const Plan *p, int64_t nt);
+// groups_beside: target groups of other sets whose calls run beside this one
 pf_status plan_exec(const Plan *p, Bump &sc, int64_t ns, const double *x, const double *y,
                     const double *g, int64_t nt, const double *xt, const double *yt,
-                    double ksigmasqr, double *vx, double *vy, int64_t nt_beside,
+                    double ksigmasqr, double *vx, double *vy, int64_t groups_beside,
                     unsigned long long *ctr, cudaEvent_t *ev, cudaStream_t st);
 // leaf level from the blob count, as the reference's level count
 int auto_level(int64_t ns, int ndirect);
