@@ -314,7 +314,7 @@ static pf_status batch_enqueue(pf_batch *b) {
             pf::Bump sc{b->slot_scratch[s], b->slot_bytes[s], 0};
             if (j.kind == 0) {
                 PF_TRY(pf::fmmx::plan_exec(b->plans[j.inst], sc, d.n, d.x, d.y, d.g, d.n, d.x, d.y,
-                                           d.ksigmasqr, d.vx, d.vy,
+                                           d.ksigmasqr, d.vx, d.vy, b->ctx->num_sms,
                                            groups - pf::fmmx::plan_groups(b->plans[j.inst], d.n),
                                            b->d_ctr + pf::fmmx::FMM_COUNTERS * s, nullptr, st));
             } else {

@@ -1182,6 +1182,7 @@ struct FmmArgs {
     double ksigmasqr, cutoff, tol;
     int ndirect;
     double *vx, *vy;
+    int num_sms;
     int64_t groups_beside = 0;  // P2P groups of other sets whose calls run beside this one
 };
 
@@ -1195,23 +1196,24 @@ static int64_t p2p_groups_expected(int64_t nblk, int64_t nt) {
 
 // Warps per target group (the result is the same), from the number of groups to
 // expect, this set's and (two thirds of) those of the sets beside it in a batch:
-// the device holds 20 one-warp CTAs per SM, and one group alone is a serial
+// the device holds 20 one-warp CTAs per SM (2960), and one group alone is a serial
 // chain of 40-100 chunks; several warps cost barriers and exchanges, 40-75% where
 // the device is full.  P2P time with 1 / 4 / 8 warps, uniform sets: 3,001 blobs 73 /
 // 42 / 30 us; 30,000 163 / 89 / 79; 38,000 87 / 81 / 93; 100,000 185 / 163 / 187;
 // 140,000 230 / 234 / 273; 150,000 198 / 280 / 325.  A call in a tree of finer
 // leaves, 62,384 blobs at level 7: 280 / 333 / 408, 15,129 at level 6: 125 / 132 / 152.
-static int p2p_warps(int64_t nblk, int64_t nt, int64_t groups_beside) {
+static int p2p_warps(int64_t nblk, int64_t nt, int64_t groups_beside, int num_sms) {
     const int64_t groups = p2p_groups_expected(nblk, nt) + 2 * groups_beside / 3;
-    return groups <= 600 ? 8 : groups <= 2200 ? 4 : 1;
+    const int64_t resident = (int64_t)num_sms * P2P_MIN_CTAS;
+    return groups <= resident / 5 ? 8 : groups <= resident * 3 / 4 ? 4 : 1;
 }
 
 // Blocks up to which each block's first group is a CTA by itself, the heaviest
-// blocks first; beyond, all groups are listed.  Uniform sets of 2^18 to 2^20 blobs
-// lose 2-4% of P2P when listed, by the order of the last CTAs.  From 65,536 blocks
-// on that is 0.3%, and the empty blocks' CTAs and the second groups being far
-// from the first cost more: 2^22 blobs in an annulus, P2P 3.10 ms, listed 2.77 (one
-// CTA per block for all its groups 2.97).
+// blocks first; beyond, all groups are listed.  Uniform sets of 150,000 and 2^20
+// blobs lose 4 and 2% of P2P when listed, by the order of the last CTAs.  From
+// 65,536 blocks on that is 0.8% (2^22 blobs), and the empty blocks' CTAs and the
+// second groups being far from the first cost more: 2^22 blobs in an annulus, P2P
+// 3.10 ms, listed 2.77 (one CTA per block for all its groups 2.97).
 constexpr int64_t P2P_DIRECT_MAX = 32768;
 
 static int64_t p2p_direct(int64_t nblk) { return nblk <= P2P_DIRECT_MAX ? nblk : 0; }
@@ -1224,10 +1226,10 @@ static int64_t p2p_more_cap(int64_t nblk, int64_t nt) {
 // CTAs for the listed groups: those of a layer around a body, or what the device
 // holds (mostly idle CTAs for every group there could be cost 13 us at 2^20
 // uniform blobs).
-static int64_t p2p_more_ctas(int64_t nblk, int64_t nt) {
-    const int64_t direct = p2p_direct(nblk);
+static int64_t p2p_more_ctas(int64_t nblk, int64_t nt, int num_sms) {
+    const int64_t direct = p2p_direct(nblk), resident = (int64_t)num_sms * P2P_MIN_CTAS;
     return std::min<int64_t>(p2p_more_cap(nblk, nt),
-                             std::max<int64_t>({148 * P2P_MIN_CTAS, nblk - direct, nt / 60 - direct}));
+                             std::max<int64_t>({resident, nblk - direct, nt / 60 - direct}));
 }
 
 static size_t fmm_scratch_bytes(const FmmCache &c, int64_t ns, int64_t nt, bool same) {
@@ -1358,12 +1360,12 @@ static pf_status exec_fmm(pf::Bump &sc, const FmmArgs &a, const FmmCache &c, dou
     if (same) T = S;  // sort_points replaced S.perm by the final permutation
 
     PF_TRY(mark(1));
-    const int warps = p2p_warps(nblk, nt, a.groups_beside);
+    const int warps = p2p_warps(nblk, nt, a.groups_beside, a.num_sms);
     auto near = [&]() -> pf_status {
         if (warps > 1) {
             PF_TRY(pf::fmmx::launch_p2p_multi(pd, warps, (unsigned)(pd.direct + more_cap), st));
         } else {
-            k_p2p<<<(unsigned)(pd.direct + p2p_more_ctas(nblk, nt)), 32, 0, st>>>(pd);
+            k_p2p<<<(unsigned)(pd.direct + p2p_more_ctas(nblk, nt, a.num_sms)), 32, 0, st>>>(pd);
             PF_TRY(pf::launch_status("k_p2p"));
         }
         return PF_OK;
@@ -1697,7 +1699,7 @@ pf_status velocity_fmm(pf_ctx *ctx, int64_t n_src, const double *x, const double
         --L;  // cutoff too large for this leaf width: coarser leaves
     }
     ctx->fmm_plan_hold = cache;  // keep the plan alive while this call's kernels run
-    FmmArgs a{n_src, n_tgt, x, y, g, xt, yt, ksigmasqr, cutoff, tol, ndirect, vx, vy};
+    FmmArgs a{n_src, n_tgt, x, y, g, xt, yt, ksigmasqr, cutoff, tol, ndirect, vx, vy, ctx->num_sms};
     stt.used_direct = 0;
     stt.leaf_level = L;
     stt.expansion_terms = np;
@@ -1819,9 +1821,9 @@ int64_t plan_groups(const Plan *p, int64_t nt) {
 
 pf_status plan_exec(const Plan *p, Bump &sc, int64_t ns, const double *x, const double *y,
                     const double *g, int64_t nt, const double *xt, const double *yt,
-                    double ksigmasqr, double *vx, double *vy, int64_t groups_beside,
+                    double ksigmasqr, double *vx, double *vy, int num_sms, int64_t groups_beside,
                     unsigned long long *ctr, cudaEvent_t *ev, cudaStream_t st) {
-    FmmArgs a{ns, nt, x, y, g, xt, yt, ksigmasqr, 0.0, 0.0, 0, vx, vy, groups_beside};
+    FmmArgs a{ns, nt, x, y, g, xt, yt, ksigmasqr, 0.0, 0.0, 0, vx, vy, num_sms, groups_beside};
     return fmm_exec(p->c, p->x0, p->y0, p->w0, sc, a, ctr, ev, nullptr, st);
 }
 

@@ -25,7 +25,7 @@ int64_t plan_groups(const Plan *p, int64_t nt);
 // groups_beside: target groups of other sets whose calls run beside this one
 pf_status plan_exec(const Plan *p, Bump &sc, int64_t ns, const double *x, const double *y,
                     const double *g, int64_t nt, const double *xt, const double *yt,
-                    double ksigmasqr, double *vx, double *vy, int64_t groups_beside,
+                    double ksigmasqr, double *vx, double *vy, int num_sms, int64_t groups_beside,
                     unsigned long long *ctr, cudaEvent_t *ev, cudaStream_t st);
 // leaf level from the blob count, as the reference's level count
 int auto_level(int64_t ns, int ndirect);
