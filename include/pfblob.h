@@ -241,7 +241,10 @@ pf_status pf_fmm_lists(int leaf_level, int block_level_drop, double root_width, 
  * (remainder <= 1e-10 of the group's share), nearer points the pair formula
  * for each panel.  Any panel order gives the same sum to that tolerance; a
  * boundary given as a chain (consecutive panels adjacent) gives the fastest.
- * Scratch: 608 B per group + 48 B per panel from the context's arena.
+ * Scratch from the context's arena: 608 B per group + 48 B per panel; from
+ * 32,768 points and 8 groups on also 5.1 MB, 608 B per four panels, 16 KB per 32
+ * groups and 28 B per point, of 2^24 points at most.  Where the arena can't grow
+ * to that, the points are taken in smaller parts, of 65,536 at least.
  * ------------------------------------------------------------------------- */
 pf_status pf_panel_velocity(pf_ctx *ctx, int64_t m, const double *gamma, const double *xs,
                             const double *ys, const double *xe, const double *ye,

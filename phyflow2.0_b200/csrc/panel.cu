@@ -304,6 +304,7 @@ constexpr int PL_P = 40;          // local expansion terms
 constexpr int64_t PL_MIN_POINTS = 32768;  // below: every group per point
 constexpr int PL_MIN_GROUPS = 8;
 constexpr int64_t PL_SLICE = (int64_t)1 << 24;  // points taken at a time
+constexpr int64_t PL_MIN_SLICE = (int64_t)1 << 16;  // .. at least, where memory is short
 // near groups on the box-grid path are summed by sub-groups of PL_SUB panels
 // (their own series where R_sub / |z - c_sub| <= PC_RHO, else the pair formula)
 constexpr int PL_SUB = 4;
@@ -839,13 +840,14 @@ static pf_status panel_velocity(pf_ctx *ctx, const char *name, int64_t m, const 
         return PF_OK;
     }
     // slices of the points: bounds the per-point scratch (28 bytes each)
-    if (n > PL_SLICE) {
-        for (int64_t i = 0; i < n; i += PL_SLICE)
+    auto sliced = [&](int64_t slice) -> pf_status {
+        for (int64_t i = 0; i < n; i += slice)
             PF_TRY(panel_velocity(ctx, name, m, gamma, xs, ys, xe, ye, cosa, sina,
-                                  std::min<int64_t>(PL_SLICE, n - i), xv + i, yv + i, vx + i, vy + i,
+                                  std::min<int64_t>(slice, n - i), xv + i, yv + i, vx + i, vy + i,
                                   accumulate, stream, source));
         return PF_OK;
-    }
+    };
+    if (n > PL_SLICE) return sliced(PL_SLICE);
     const int64_t ngroups = pf::ceil_div(m, PC_G);
     const size_t gbytes = sizeof(PanelGroup) * (size_t)ngroups;
     const size_t pbytes = sizeof(PanelSm) * (size_t)m;
@@ -863,13 +865,19 @@ static pf_status panel_velocity(pf_ctx *ctx, const char *name, int64_t m, const 
     const size_t ibytes = boxed ? sizeof(int32_t) * (size_t)n : 0;
     const int64_t nsubs = pf::ceil_div(m, (int64_t)PL_SUB);
     const size_t sbytes = boxed ? sizeof(PanelGroup) * (size_t)nsubs : 0;
-    PF_TRY(pf::arena_reserve(ctx, pf::align256(gbytes) + pf::align256(pbytes) +
-                                      (boxed ? pf::align256(sizeof(PanelGrid)) +
-                                                   pf::align256(lbytes) + pf::align256(mbytes) +
-                                                   pf::align256(fbytes) + pf::align256(sbytes) +
-                                                   pf::align256(wbytes) + pf::align256(qbytes) +
-                                                   pf::align256(ibytes)
-                                             : 0)));
+    const pf_status room =
+        pf::arena_reserve(ctx, pf::align256(gbytes) + pf::align256(pbytes) +
+                                   (boxed ? pf::align256(sizeof(PanelGrid)) + pf::align256(lbytes) +
+                                                pf::align256(mbytes) + pf::align256(fbytes) +
+                                                pf::align256(sbytes) + pf::align256(wbytes) +
+                                                pf::align256(qbytes) + pf::align256(ibytes)
+                                          : 0));
+    // no memory for the points' scratch: slices of a quarter, down to 64k points
+    if (room == PF_ERR_OOM && boxed && n > PL_MIN_SLICE) {
+        pf::clear_error();
+        return sliced(std::max<int64_t>(pf::ceil_div(n, 4), PL_MIN_SLICE));
+    }
+    PF_TRY(room);
     auto *groups = static_cast<PanelGroup *>(pf::arena_take(ctx, gbytes));
     auto *pan = static_cast<PanelSm *>(pf::arena_take(ctx, pbytes));
     PanelGrid *gd = nullptr;

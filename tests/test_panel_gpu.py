@@ -225,3 +225,66 @@ def test_box_order_gives_the_input_orders_values(n, m):
                                    xv[:2000].copy(), yv[:2000].copy())
     inv = np.argsort(order)[:2000]
     assert normwise_err(ax.cpu().numpy()[inv], ay.cpu().numpy()[inv], rx, ry) <= TOL
+
+
+def _ring_points(n, seed):
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    r = 1.0 + 0.5 * torch.rand(n, dtype=torch.float64, device="cuda", generator=gen)
+    a = 6.283185307179586 * torch.rand(n, dtype=torch.float64, device="cuda", generator=gen)
+    return r * torch.cos(a), r * torch.sin(a)
+
+
+def test_more_points_than_one_part():
+    """Above 2^24 points the set is taken in parts: bitwise the parts' own calls,
+    also accumulated."""
+    import pfblob
+    from pfblob import workloads as wl
+    ps = wl.cylinder_panels(128)
+    arrs = [torch.from_numpy(np.ascontiguousarray(a)).cuda()
+            for a in (ps.gamma, ps.xs, ps.ys, ps.xe, ps.ye, ps.cosa, ps.sina)]
+    part = 1 << 24
+    x, y = _ring_points(part + 40001, 24)
+    vx, vy = torch.ones_like(x), torch.full_like(y, -2.0)
+    pfblob.panel_velocity_device(*arrs, x, y, vx, vy, accumulate=True)
+    for k in (slice(0, part), slice(part, None)):
+        ax, ay = pfblob.inducedVelocity(*arrs, x[k], y[k])
+        assert torch.equal(vx[k], ax + 1.0) and torch.equal(vy[k], ay - 2.0)
+
+
+def test_points_in_parts_where_memory_is_short():
+    """4 million points need 117 MB of scratch; with 48 MB free they are taken in
+    smaller parts, to the same values within the gate, and no error is left."""
+    import threading
+    import pfblob
+    from pfblob import _lib
+    from pfblob import workloads as wl
+    ps = wl.cylinder_panels(128)
+    arrs = [torch.from_numpy(np.ascontiguousarray(a)).cuda()
+            for a in (ps.gamma, ps.xs, ps.ys, ps.xe, ps.ye, ps.cosa, ps.sina)]
+    x, y = _ring_points(1 << 22, 22)
+    rx, ry = pfblob.inducedVelocity(*arrs, x, y)
+    vx, vy = torch.zeros_like(x), torch.zeros_like(y)
+    out = {}
+
+    def run():  # a thread's context has a scratch arena of its own
+        try:
+            pfblob.panel_velocity_device(*arrs, x[:40000], y[:40000], vx[:40000], vy[:40000])
+            torch.cuda.synchronize()
+            _lib.check(_lib.lib.pf_trim(_lib.context(0)))
+            torch.cuda.empty_cache()
+            fill = torch.empty(torch.cuda.mem_get_info()[0] - (48 << 20), dtype=torch.uint8,
+                               device="cuda")
+            pfblob.panel_velocity_device(*arrs, x, y, vx, vy)
+            torch.cuda.synchronize()
+            out["error"] = _lib.lib.pf_last_error()
+            del fill
+        except Exception as e:  # noqa: BLE001 (shown by the assertion below)
+            out["raised"] = e
+
+    t = threading.Thread(target=run)
+    t.start()
+    t.join()
+    torch.cuda.empty_cache()
+    assert out == {"error": b""}, out
+    assert normwise_err(vx.cpu().numpy(), vy.cpu().numpy(), rx.cpu().numpy(),
+                        ry.cpu().numpy()) <= TOL
