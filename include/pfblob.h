@@ -526,7 +526,9 @@ pf_status pf_moments(pf_ctx *ctx, int64_t n, const double *x, const double *y,
  * velocity of every instance at its own blobs, then optionally its remesh --
  * into one CUDA graph; pf_batch_run replays it with one graph launch on
  * `stream`.  Direct-sum instances run together in one persistent kernel;
- * FMM and remesh jobs run on library streams inside the graph.  The batch
+ * FMM and remesh jobs run on n_streams library streams each inside the graph
+ * (one stream: one job at a time), with scratch for the largest job of each
+ * stream; where memory for the remeshes' own is short, on n_streams in all.  The batch
  * keeps the instance pointers: inputs may change in value between runs but
  * not in size (create a new batch when sizes change).  Results are the same
  * as the single-instance calls with the same method and tree.

@@ -125,6 +125,37 @@ static void batch_free(pf_batch *b) {
     delete b;
 }
 
+// Distribute the jobs, longest first, over F slots, the remeshes over the S - F
+// slots beyond if there are any, and allocate the slots' scratch.
+static pf_status batch_slots(pf_batch *b, const std::vector<Job> &jobs, int F, int S) {
+    for (auto p : b->slot_scratch) cudaFree(p);
+    b->nstreams = S;
+    b->slot_jobs.assign(S, {});
+    b->slot_scratch.assign(S, nullptr);
+    b->slot_bytes.assign(S, 0);
+    std::vector<double> load(S, 0.0);
+    for (const Job &j : jobs) {
+        const bool own = j.kind == 1 && S > F;
+        const auto lo = load.begin() + (own ? F : 0);
+        const auto hi = own ? load.end() : load.begin() + F;
+        const int s = (int)(std::min_element(lo, hi) - load.begin());
+        load[s] += j.cost;
+        b->slot_jobs[s].push_back(j);
+    }
+    for (int s = 0; s < S; ++s) {
+        size_t mx = 4096;
+        for (const Job &j : b->slot_jobs[s]) mx = std::max(mx, j.scratch);
+        b->slot_bytes[s] = mx;
+        cudaError_t e = cudaMalloc(&b->slot_scratch[s], mx);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            pf::set_error("pf_batch_create: scratch allocation of %zu bytes failed", mx);
+            return PF_ERR_OOM;
+        }
+    }
+    return PF_OK;
+}
+
 static pf_status batch_build(pf_batch *b, double tol) {
     pf_ctx *ctx = b->ctx;
     const int n = b->n;
@@ -255,31 +286,19 @@ static pf_status batch_build(pf_batch *b, double tol) {
                      [](const Job &a, const Job &c) { return a.cost > c.cost; });
     int64_t n_rm = 0;
     for (const Job &j : jobs) n_rm += j.kind == 1;
-    const int F = b->nstreams, S = F > 1 ? F + (int)std::min<int64_t>(n_rm, F) : F;
-    b->nstreams = S;
-    b->slot_jobs.assign(S, {});
-    std::vector<double> load(S, 0.0);
-    for (const Job &j : jobs) {
-        const bool own = j.kind == 1 && S > F;
-        const auto lo = load.begin() + (own ? F : 0);
-        const auto hi = own ? load.end() : load.begin() + F;
-        const int s = (int)(std::min_element(lo, hi) - load.begin());
-        load[s] += j.cost;
-        b->slot_jobs[s].push_back(j);
+    const int F = b->nstreams;
+    const int own_slots = F > 1 ? (int)std::min<int64_t>(n_rm, F) : 0;
+    pf_status room = batch_slots(b, jobs, F, F + own_slots);
+    // no memory for the remeshes' slots, or none left for the graph: all jobs in
+    // the others
+    size_t free_bytes = 0, all_bytes = 0;
+    PF_CUDA_TRY(cudaMemGetInfo(&free_bytes, &all_bytes));
+    if (own_slots > 0 && (room == PF_ERR_OOM || free_bytes < ((size_t)64 << 20))) {
+        room = batch_slots(b, jobs, F, F);
+        if (room == PF_OK) pf::clear_error();
     }
-    b->slot_scratch.assign(S, nullptr);
-    b->slot_bytes.assign(S, 0);
-    for (int s = 0; s < S; ++s) {
-        size_t mx = 4096;
-        for (const Job &j : b->slot_jobs[s]) mx = std::max(mx, j.scratch);
-        b->slot_bytes[s] = mx;
-        cudaError_t e = cudaMalloc(&b->slot_scratch[s], mx);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            pf::set_error("pf_batch_create: scratch allocation of %zu bytes failed", mx);
-            return PF_ERR_OOM;
-        }
-    }
+    PF_TRY(room);
+    const int S = b->nstreams;
     PF_CUDA_TRY(cudaMalloc(&b->d_ctr, sizeof(unsigned long long) * pf::fmmx::FMM_COUNTERS * std::max(1, S)));
     PF_CUDA_TRY(cudaMalloc(&b->d_totals, sizeof(int32_t) * std::max(1, n)));
     PF_CUDA_TRY(cudaMalloc(&b->d_bads, sizeof(int32_t) * std::max(1, n)));

@@ -146,3 +146,39 @@ def test_remeshes_on_streams_of_their_own(streams, remesh):
                 assert torch.equal(xn, r["x"]) and torch.equal(yn, r["y"])
                 assert torch.equal(gn, r["g"])
     bt.close()
+
+
+def test_remesh_streams_where_memory_is_short():
+    """With 100 MB less free than the batch takes, the remeshes share the FMM's
+    streams and scratch: bitwise the same results."""
+    from pfblob import workloads as wl
+    from pfblob.batch import Batch
+    sims = []
+    for i in range(8):
+        b = wl.uniform_square(n=400000, sigma=0.003, instance=i)
+        sims.append({"x": T(b.x), "y": T(b.y), "g": T(b.g), "sigma": b.sigma})
+    kw = dict(tol=1e-6, n_streams=8, methods=[0] * 8, leaf_levels=[7] * 8)
+
+    def outside_torch():
+        free, total = torch.cuda.mem_get_info()
+        return total - free - torch.cuda.memory_reserved()
+
+    bt = Batch(sims, **kw)
+    bt.run()
+    want = [{k: r[k].clone() for k in ("vx", "vy", "x", "y", "g")} for r in bt.results()]
+    bt.close()
+    del bt  # its tensors stay in torch's cache, for the next batch
+    before = outside_torch()
+    bt = Batch(sims, **kw)
+    taken = outside_torch() - before
+    bt.close()
+    del bt
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - taken + (100 << 20), dtype=torch.uint8,
+                       device=DEV)
+    bt = Batch(sims, **kw)
+    bt.run()
+    got = bt.results()
+    assert all(torch.equal(p[k], q[k]) for p, q in zip(want, got) for k in p)
+    bt.close()
+    del fill
+    torch.cuda.empty_cache()
