@@ -334,7 +334,7 @@ __global__ void k_panel_grid_init(PanelGrid *gd) {
     gd->sorted = 0;
 }
 
-// min / max of the point coordinates (order-preserving integer images)
+// min / max of the finite points' coordinates (order-preserving integer images)
 __global__ void __launch_bounds__(PN_THREADS)
 k_panel_bbox(int64_t n, const double *__restrict__ xv, const double *__restrict__ yv,
              PanelGrid *gd) {
@@ -351,6 +351,7 @@ k_panel_bbox(int64_t n, const double *__restrict__ xv, const double *__restrict_
         }
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
+            if (!isfinite(xs4[u]) || !isfinite(ys4[u])) continue;
             const unsigned long long ox = pl_ord(xs4[u]), oy = pl_ord(ys4[u]);
             mnx = min(mnx, ox);
             mxx = max(mxx, ox);
@@ -534,8 +535,7 @@ __global__ void k_panel_grid_set(PanelGrid *gd) {
     const double x0 = pl_unord(gd->mn[0]), x1 = pl_unord(gd->mx[0]);
     const double y0 = pl_unord(gd->mn[1]), y1 = pl_unord(gd->mx[1]);
     double e = fmax(x1 - x0, y1 - y0);
-    // non-finite coordinates give no usable grid: one box holding everything
-    // would be near every group, i.e. the per-point path
+    // (no finite point, all in one place, or farther apart than the range: any grid)
     if (!(e > 0.0) || !isfinite(e)) e = 1.0;
     gd->x0 = isfinite(x0) ? x0 : 0.0;
     gd->y0 = isfinite(y0) ? y0 : 0.0;

@@ -288,3 +288,26 @@ def test_points_in_parts_where_memory_is_short():
     assert out == {"error": b""}, out
     assert normwise_err(vx.cpu().numpy(), vy.cpu().numpy(), rx.cpu().numpy(),
                         ry.cpu().numpy()) <= TOL
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), -float("inf")])
+def test_points_that_are_not_finite_leave_the_others_alone(bad):
+    """In a large set too, a point that is not finite changes no other point's
+    velocity (bitwise), and its own is not finite."""
+    import pfblob
+    from pfblob import workloads as wl
+    ps = wl.cylinder_panels(128)
+    arrs = [torch.from_numpy(np.ascontiguousarray(a)).cuda()
+            for a in (ps.gamma, ps.xs, ps.ys, ps.xe, ps.ye, ps.cosa, ps.sina)]
+    x, y = _ring_points(40000, 40)
+    x[0], y[0], x[1], y[1] = -1.5, -1.5, 1.5, 1.5  # the others' box
+    vx, vy = pfblob.inducedVelocity(*arrs, x, y)
+    idx = [7, 20000, 39999]
+    rest = torch.ones(40000, dtype=torch.bool, device="cuda")
+    rest[idx] = False
+    x[idx[0]] = bad
+    y[idx[1]] = bad
+    x[idx[2]] = y[idx[2]] = bad
+    wx, wy = pfblob.inducedVelocity(*arrs, x, y)
+    assert torch.equal(vx[rest], wx[rest]) and torch.equal(vy[rest], wy[rest])
+    assert not torch.isfinite(wx[~rest] + wy[~rest]).any()
