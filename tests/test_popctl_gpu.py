@@ -144,3 +144,20 @@ def test_fused_control_in_a_wide_window(side):
         rx, ry, rg = pfblob.remesh_device(*t, h, -1.5 * h, -1.5 * h)
         px, py, pg, pt = pfblob.population_control_device(rx, ry, rg, *thr)
         assert torch.equal(fx, px) and torch.equal(fy, py) and torch.equal(fg, pg) and ft == pt
+
+
+def test_population_control_of_more_than_33_million():
+    """Above 2^25 values the scan of the kept flags takes its launch for the tiles'
+    totals: against torch on the device."""
+    import pfblob
+    n = (1 << 25) + 4097
+    gen = torch.Generator(device="cuda").manual_seed(25)
+    x = torch.rand(n, dtype=torch.float64, device="cuda", generator=gen)
+    y = torch.rand(n, dtype=torch.float64, device="cuda", generator=gen)
+    g = torch.randn(n, dtype=torch.float64, device="cuda", generator=gen)
+    thr, limit = 0.5, 1e9  # the loss is admissible at the first threshold
+    xo, yo, go, used = pfblob.population_control_device(x, y, g, thr, limit)
+    keep = g.abs() >= thr
+    assert used == thr and xo.numel() == int(keep.sum())
+    for a, b in ((xo, x), (yo, y), (go, g)):
+        assert torch.equal(a, b[keep])
