@@ -4,7 +4,7 @@
 // synchronisation.  A serving loop makes one call per request instead of a
 // dozen small ones.  pf_step_graph_* capture that call once into a CUDA graph
 // and replay it with one graph launch per step (no launch gaps between the
-// step's ~35 kernels and memsets).
+// step's ~25 kernels and the memsets).
 #include <cmath>
 #include <new>
 
